@@ -5,13 +5,14 @@
 // computed by one fixed recipe, whatever n is and wherever the row lies in the
 // batch, so a row's result is the same bits however the tokens are cut into
 // steps: k is cut into segments of SEG values at fixed places; within a segment
-// the products are added by one chain of fmaf in ascending order from zero; the
-// segments' sums are added in ascending order.  Two kernels follow the recipe:
-// one for many tokens (a thread walks all segments of its outputs) and one for
-// the few tokens of a decode step (a block per segment, so that a narrow matrix
-// still keeps every SM's loads in flight; the segments' sums go through scratch
-// and a second kernel adds them in order).  A and W are float or bfloat16
-// (widened exactly); no reduced-precision matrix mode is involved.
+// the products of even k and of odd k are added by one chain of fmaf each, in
+// ascending order from zero, and the two sums are added; the segments' sums are
+// added in ascending order.  One kernel follows the recipe for every shape: a
+// block walks one or more segments of a tile of rows and features.  Where tiles
+// alone leave the SMs without work, the segments are shared out over blocks, which
+// leave their sums in scratch for a second kernel that adds them in order.
+// A and W are float or bfloat16 (widened exactly); no reduced-precision matrix
+// mode is involved.
 //
 // The reference computes y = W x with rows of W as output features
 // (src/llm/model_load.c:452, src/llm/model_attn.c:234-255); its products are
@@ -21,209 +22,326 @@
 
 namespace jb {
 
-constexpr int BM = 64, BN = 64, BK = 16;
-constexpr int SEG = 512;      // k per segment; a multiple of BK and of SK_K
+constexpr int BK = 64;        // k of a stage
+constexpr int SEG = 512;      // k of a segment
+static_assert(SEG % BK == 0, "segments end where stages end");
+// values a row of a stage takes in shared memory: a multiple of 16 bytes, and neighbouring rows start in other banks
+template <typename T> constexpr int ROW = BK + 16 / (int)sizeof(T);
 
-template <typename T>
-__device__ __forceinline__ void load4(const T *base, size_t row, int rows, int col, int k,
-                                      bool vec, float *v)
+// Two floats side by side, and one multiply-add of both (each rounded like fmaf).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
 {
-    v[0] = v[1] = v[2] = v[3] = 0.0f;
-    if ((int)row >= rows)
-        return;
-    const T *p = base + row * (size_t)k + col;
-    if (vec && col + 3 < k) {
-        if constexpr (sizeof(T) == 4) {
-            float4 f = *reinterpret_cast<const float4 *>(p);
-            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-        } else {
-            uint2 u = *reinterpret_cast<const uint2 *>(p);
-            v[0] = __uint_as_float(u.x << 16);
-            v[1] = __uint_as_float(u.x & 0xffff0000u);
-            v[2] = __uint_as_float(u.y << 16);
-            v[3] = __uint_as_float(u.y & 0xffff0000u);
-        }
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        if (col + i < k)
-            v[i] = to_f(p[i]);
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float sum2(f32x2 v)
+{
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
 }
 
-template <typename TA, typename TW>
-__global__ void __launch_bounds__(256)
-gemm_simt_kernel(const TA *__restrict__ A, const TW *__restrict__ W, float *__restrict__ out,
-                 int n, int m, int k, bool vec)
+// Four consecutive values of a row in shared memory as two pairs.
+__device__ __forceinline__ void pairs(const float *p, f32x2 &lo, f32x2 &hi)
 {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
+    ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
+    lo = v.x;
+    hi = v.y;
+}
+__device__ __forceinline__ void pairs(const bf16 *p, f32x2 &lo, f32x2 &hi)
+{
+    uint2 u = *reinterpret_cast<const uint2 *>(p);
+    lo = (f32x2)(u.x & 0xffff0000u) << 32 | u.x << 16;
+    hi = (f32x2)(u.y & 0xffff0000u) << 32 | u.y << 16;
+}
+
+// Asks for ROWS rows of BK values from k0 on, src[row0 + r][k0 ..], to be put into a stage.
+// Rows from `have` on and values from kb on become zeros.  vec: 16 bytes at a time, asynchronously.
+template <typename T, int ROWS, int THREADS>
+__device__ __forceinline__ void fetch(T *stage, const T *__restrict__ src, long long row0, int have, int k,
+                                      int k0, int kb, bool vec)
+{
+    constexpr int V = 16 / sizeof(T), PER = BK / V;
+    if (vec) {
+#pragma unroll
+        for (int i0 = 0; i0 < ROWS * PER; i0 += THREADS) {
+            int i = i0 + threadIdx.x;
+            if (ROWS * PER % THREADS && i >= ROWS * PER)
+                break;
+            int r = i / PER, c = (i % PER) * V;
+            bool in = row0 + r < have && k0 + c < kb;
+            const T *p = in ? src + (row0 + r) * (size_t)k + k0 + c : src;
+            uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + r * ROW<T> + c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(p), "r"(in ? 16 : 0)
+                         : "memory");
+        }
+    } else {
+        for (int i = threadIdx.x; i < ROWS * BK; i += THREADS) {
+            int r = i / BK, c = i % BK;
+            stage[r * ROW<T> + c] = row0 + r < have && k0 + c < kb ? src[(row0 + r) * (size_t)k + k0 + c] : from_f<T>(0.0f);
+        }
+    }
+}
+
+// A block's threads stand TX along the features and TY along the rows; a thread owns the rows
+// ty + TY i (i < RT) and the features tx + TX j (j < CT) of the block's tile.  Along k, four values of a row
+// or feature come out of shared memory in one access and feed CT or RT pairs of multiply-adds.
+// KEEP: the sum over the segments stays in registers (else in shared memory, each thread its own).
+template <int RT, int CT, int TX, int TY, int ST> struct SimtTile {
+    static constexpr int R = RT, C = CT, X = TX, Y = TY, STAGES = ST;
+    static constexpr bool KEEP = RT * CT <= 16;
+    static constexpr int ROWS = RT * TY, FEATS = CT * TX, THREADS = TX * TY;
+    template <typename TA, typename TW> static constexpr int smem()
+    {
+        return ST * (ROW<TA> * ROWS * (int)sizeof(TA) + ROW<TW> * FEATS * (int)sizeof(TW)) + (KEEP ? 0 : ROWS * FEATS * 4);
+    }
+};
+
+// grid: x row tiles and feature tiles, the row tiles next to each other (so that the blocks that read the
+// same weights run at the same time), z groups of segments.  With one group the sums of a block's
+// segments stay with its threads and `out` is the result; else each segment's sums go to
+// out[segment][n][m].
+template <typename TA, typename TW, typename Tile, bool PARTS>
+__global__ void __launch_bounds__(Tile::THREADS, Tile::ROWS == 64 ? 2 : 1)
+gemm_simt_kernel(const TA *A, const TW *__restrict__ W, float *__restrict__ out, int n, int m, int k, int row_tiles,
+                 bool vec, bool early)
+{
+    constexpr int RT = Tile::R, CT = Tile::C, TX = Tile::X, TY = Tile::Y, ST = Tile::STAGES, THREADS = Tile::THREADS;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TW *Ws = reinterpret_cast<TW *>(smem_raw);
+    TA *As = reinterpret_cast<TA *>(Ws + ST * ROW<TW> * Tile::FEATS);
+    float *Ts = reinterpret_cast<float *>(As + ST * ROW<TA> * Tile::ROWS);
     pdl_trigger();
-    pdl_wait();
     int tid = threadIdx.x;
-    int tx = tid % 16, ty = tid / 16;
-    size_t n0 = (size_t)blockIdx.y * BM, m0 = (size_t)blockIdx.x * BN;
-    int lr = tid / 4, lc = (tid % 4) * 4;  // this thread's 4 values of a 64 x 16 tile
-
-    float acc[4][4], total[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            acc[i][j] = total[i][j] = 0.0f;
-
-    // the next tile's values are on their way while this tile is multiplied
-    float a4[4], w4[4];
-    load4<TA>(A, n0 + lr, n, lc, k, vec, a4);
-    load4<TW>(W, m0 + lr, m, lc, k, vec, w4);
-    for (int k0 = 0; k0 < k; k0 += BK) {
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            As[lc + i][lr] = a4[i];
-            Ws[lc + i][lr] = w4[i];
-        }
-        __syncthreads();
-        if (k0 + BK < k) {
-            load4<TA>(A, n0 + lr, n, k0 + BK + lc, k, vec, a4);
-            load4<TW>(W, m0 + lr, m, k0 + BK + lc, k, vec, w4);
-        }
-#pragma unroll
-        for (int kk = 0; kk < BK; kk++) {
-            float a[4], w[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                a[i] = As[kk][ty * 4 + i];
-                w[i] = Ws[kk][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-        }
-        if ((k0 + BK) % SEG == 0 || k0 + BK >= k) {
-            // a segment ends: its sum joins the total; the first one is the total
-            bool first = k0 < SEG;
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    total[i][j] = first ? acc[i][j] : total[i][j] + acc[i][j];
-                    acc[i][j] = 0.0f;
-                }
-        }
+    // a warp's lanes stand eight along the features and four along the rows where both run, lane bits
+    // 0, 2, 4 and 1, 3: neighbours (i ^ 1, i ^ 2) then ask for the same 16 bytes, and an access to shared
+    // memory takes fewer turns
+    int tx, ty;
+    if constexpr (TY % 4 == 0) {
+        int w = tid >> 5, l = tid & 31;
+        tx = ((l & 1) | (l >> 1 & 2) | (l >> 2 & 4)) + 8 * (w % (TX / 8));
+        ty = ((l >> 1 & 1) | (l >> 2 & 2)) + 4 * (w / (TX / 8));
+    } else {
+        tx = tid % TX;
+        ty = tid / TX;
     }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        size_t r = n0 + ty * 4 + i;
-        if (r >= (size_t)n)
-            continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            size_t c = m0 + tx * 4 + j;
-            if (c < (size_t)m)
-                out[r * m + c] = total[i][j];
-        }
-    }
-}
-
-// The same recipe for up to 16 tokens (a decode step): a block takes 128 features,
-// all tokens and ONE segment of k, and writes the segment's sums to `part`
-// [segments, n, m]; a thread owns four features and four tokens (16 chains of
-// fmaf), so that a value read from shared memory feeds four multiply-adds.  With one
-// segment in all, the sums are the result and go to `out` directly.
-constexpr int SK_FEATS = 128, SK_K = 32, SK_THREADS = 128, SK_MAX_N = 16;
-static_assert(SEG % BK == 0 && SEG % SK_K == 0, "segments end where both kernels' tiles end");
-
-template <typename TA, typename TW>
-__global__ void __launch_bounds__(SK_THREADS)
-gemm_simt_skinny_kernel(const TA *__restrict__ A, const TW *__restrict__ W, float *__restrict__ part,
-                        int n, int m, int k, bool vec)
-{
-    __shared__ __align__(16) float Ws[SK_K][SK_FEATS + 4];
-    __shared__ __align__(16) float As[SK_K][SK_MAX_N + 4];
-    pdl_trigger();
-    pdl_wait();
-    int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int fx = lane, g = warp;                             // features 4 fx .. 4 fx + 3, tokens 4 g .. 4 g + 3
-    size_t m0 = (size_t)blockIdx.x * SK_FEATS;
-    int ka = blockIdx.y * SEG, kb = min(k, ka + SEG);    // this block's segment
-    // loads of a 128 x 32 weight tile: rows lane + 32 j, the warp's quarter of k;
-    // of the 16 x 32 token tile: row tid % 16, four values of k
-    int wk = warp * 8, ar = tid & 15, ak = (tid >> 4) * 4;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            acc[i][j] = 0.0f;
-    float w4[4][2][4], a4[4];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-                load4<TW>(W, m0 + lane + 32 * j, m, k0 + wk + 4 * h, k, vec, w4[j][h]);
-        load4<TA>(A, (size_t)ar, n, k0 + ak, k, vec, a4);
+    long long n0 = (long long)(blockIdx.x % row_tiles) * Tile::ROWS, m0 = (long long)(blockIdx.x / row_tiles) * Tile::FEATS;
+    int segments = (k + SEG - 1) / SEG;
+    int s0 = (int)((long long)segments * blockIdx.z / gridDim.z);
+    int s1 = (int)((long long)segments * (blockIdx.z + 1) / gridDim.z);
+    int ka = s0 * SEG, kb = min(k, s1 * SEG);
+    int steps = (kb - ka + BK - 1) / BK;
+    auto fetch_w = [&](int s) {
+        fetch<TW, Tile::FEATS, THREADS>(Ws + (s % ST) * ROW<TW> * Tile::FEATS, W, m0, m, k, ka + s * BK, kb, vec);
     };
-    fetch(ka);
-    for (int k0 = ka; k0 < kb; k0 += SK_K) {
-        __syncthreads();
+    auto fetch_a = [&](int s) {
+        fetch<TA, Tile::ROWS, THREADS>(As + (s % ST) * ROW<TA> * Tile::ROWS, A, n0, n, k, ka + s * BK, kb, vec);
+    };
+    // early: the first stages' weights are on their way while the kernel before this one ends
+    if (!early)
+        pdl_wait();
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+    for (int s = 0; s < ST - 1; s++)
+        if (s < steps)
+            fetch_w(s);
+    if (early)
+        pdl_wait();
 #pragma unroll
-            for (int h = 0; h < 2; h++)
+    for (int s = 0; s < ST - 1; s++) {
+        if (s < steps)
+            fetch_a(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    f32x2 acc[RT][CT];
+    float total[Tile::KEEP ? RT : 1][Tile::KEEP ? CT : 1];
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-                    Ws[wk + 4 * h + i][lane + 32 * j] = w4[j][h][i];
+    for (int i = 0; i < RT; i++)
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-            As[ak + i][ar] = a4[i];
-        __syncthreads();
-        if (k0 + SK_K < kb)
-            fetch(k0 + SK_K);
+        for (int j = 0; j < CT; j++) {
+            acc[i][j] = 0;
+            if (Tile::KEEP)
+                total[i][j] = 0.0f;
+        }
+    for (int s = 0; s < steps; s++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();                 // stage s is there for all, and all are done with stage s - 1
+        if (s + ST - 1 < steps) {
+            fetch_w(s + ST - 1);
+            fetch_a(s + ST - 1);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const TW *ws = Ws + (s % ST) * ROW<TW> * Tile::FEATS + tx * ROW<TW>;
+        const TA *as = As + (s % ST) * ROW<TA> * Tile::ROWS + ty * ROW<TA>;
 #pragma unroll
-        for (int kk = 0; kk < SK_K; kk++) {
-            float4 w = *reinterpret_cast<const float4 *>(&Ws[kk][4 * fx]);
-            float4 a = *reinterpret_cast<const float4 *>(&As[kk][4 * g]);
-            float wv[4] = {w.x, w.y, w.z, w.w}, av[4] = {a.x, a.y, a.z, a.w};
+        for (int kk = 0; kk < BK; kk += 4) {
+            f32x2 w0[CT], w1[CT];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int j = 0; j < CT; j++)
+                pairs(ws + j * TX * ROW<TW> + kk, w0[j], w1[j]);
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    acc[i][j] = fmaf(av[j], wv[i], acc[i][j]);
+            for (int i = 0; i < RT; i++) {
+                f32x2 a0, a1;
+                pairs(as + i * TY * ROW<TA> + kk, a0, a1);
+#pragma unroll
+                for (int j = 0; j < CT; j++)
+                    acc[i][j] = fma2(a0, w0[j], acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < CT; j++)
+                    acc[i][j] = fma2(a1, w1[j], acc[i][j]);
+            }
+        }
+        if ((s + 1) % (SEG / BK) == 0 || s + 1 == steps) {
+            // a segment ends
+            int seg = s0 + s / (SEG / BK);
+#pragma unroll
+            for (int i = 0; i < RT; i++) {
+                long long r = n0 + ty + TY * i;
+#pragma unroll
+                for (int j = 0; j < CT; j++) {
+                    float v = sum2(acc[i][j]);
+                    acc[i][j] = 0;
+                    if (PARTS) {
+                        long long c = m0 + tx + TX * j;
+                        if (r < n && c < m)
+                            out[((size_t)seg * n + r) * m + c] = v;
+                    } else if (Tile::KEEP) {
+                        total[i][j] = seg == 0 ? v : total[i][j] + v;
+                    } else {
+                        float *t = Ts + (i * CT + j) * THREADS + tid;
+                        *t = seg == 0 ? v : *t + v;
+                    }
+                }
+            }
         }
     }
-    float *dst = part + (size_t)blockIdx.y * n * m;
+    if (!PARTS) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        int r = 4 * g + j;
-        if (r >= n)
-            continue;
+        for (int i = 0; i < RT; i++) {
+            long long r = n0 + ty + TY * i;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            size_t c = m0 + 4 * fx + i;
-            if (c < (size_t)m)
-                dst[(size_t)r * m + c] = acc[i][j];
+            for (int j = 0; j < CT; j++) {
+                long long c = m0 + tx + TX * j;
+                if (r < n && c < m)
+                    out[(size_t)r * m + c] = Tile::KEEP ? total[i][j] : Ts[(i * CT + j) * THREADS + tid];
+            }
         }
     }
 }
 
-// out = ((part[0] + part[1]) + part[2]) + ...: the segments' sums in ascending order.
+// out = ((part[0] + part[1]) + part[2]) + ...: the segments' sums in ascending order, V
+// neighbours a thread.
+template <int V>
 __global__ void __launch_bounds__(256)
-gemm_simt_join_kernel(const float *__restrict__ part, float *__restrict__ out, long long count,
-                      int segments)
+gemm_simt_join_kernel(const float *part, float *__restrict__ out, long long count, int segments)
 {
     pdl_trigger();
     pdl_wait();
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (i >= count)
         return;
-    float t = part[i];
-    for (int s = 1; s < segments; s++)
-        t = t + part[(size_t)s * count + i];
-    out[i] = t;
+    if constexpr (V == 4) {
+        float4 t = load4(part + i);
+        for (int s = 1; s < segments; s += 4) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (s + u < segments)
+                    v[u] = load4(part + (size_t)(s + u) * count + i);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (s + u < segments) {
+                    t.x += v[u].x;
+                    t.y += v[u].y;
+                    t.z += v[u].z;
+                    t.w += v[u].w;
+                }
+        }
+        store4(out + i, t);
+    } else {
+        float t = part[i];
+        for (int s = 1; s < segments; s++)
+            t = t + part[(size_t)s * count + i];
+        out[i] = t;
+    }
+}
+
+// Which tile: rows up to 8, 16 and 32 stand in one tile, so that a weight is read once; more rows in tiles of 64.
+//
+// Up to 16 rows the weights' bytes are the bound.  A narrow tile (64 features) keeps many blocks on an SM, each
+// with two stages of 16 KB on their way; every multiply-add takes its weight from shared memory, and the reads of
+// weights (twice per block of 8 rows) are what is fullest.  From 32 rows on the multiply-adds are the bound
+// (72.7 TFLOP/s is what this instruction gives); four to eight rows and four features a thread, the stage
+// unrolled whole, were the fastest of the tiles tried: 8 x 8 a thread spills, more blocks of fewer registers
+// lose more to waiting than they hide.
+// One B200, float, microseconds (before: blocks of 64 x 64 with 16 values of k a stage, or of 128 features and
+// 16 rows), with the second kernel where k is shared out:
+//   rows 8:   6144 x 2560  18.0 (76.7)   2560 x 4096  13.5 (92.3)   19456 x 2560  49 (112)   151936 x 2560  271 (703)
+//   rows 16:  6144 x 2560  23.0          2560 x 4096  19.2          19456 x 2560  68         151936 x 2560  406
+//   rows 64:  6144 x 2560  70 (166)      2560 x 4096  47 (202)      19456 x 2560  211 (375)  2560 x 9728  121 (475)
+//   rows 300: 6144 x 2560  277 (384)     2560 x 4096  178 (313)     19456 x 2560  742 (1089) 2560 x 9728  426 (738)
+// and 2,048 rows run at 45 TFLOP/s (31).  The error against 64 bits is 2.9e-7 of the result (4.1e-7): a chain is
+// half as long.
+typedef SimtTile<4, 2, 32, 2, 3> Rows8;
+typedef SimtTile<4, 4, 16, 4, 3> Rows16;
+typedef SimtTile<8, 4, 32, 4, 2> Rows32;
+typedef SimtTile<8, 4, 16, 8, 2> Rows64;
+static_assert(Rows8::FEATS == Rows64::FEATS && Rows16::FEATS == Rows64::FEATS, "simt_groups counts so");
+
+static int simt_segments(int k) { return (k + SEG - 1) / SEG; }
+
+// Groups of segments: as few as give every SM a few blocks (four small ones, or two of the others).  The sums
+// that pass through scratch cost 8 bytes a segment, row and feature, the weights 4 bytes x 512 a segment and
+// feature.
+static int simt_groups(int n, int m, int k)
+{
+    int rows = n <= 8 ? Rows8::ROWS : n <= 16 ? Rows16::ROWS : n <= 32 ? Rows32::ROWS : Rows64::ROWS;
+    int feats = n <= 32 && n > 16 ? Rows32::FEATS : Rows64::FEATS;
+    long long tiles = ((long long)m + feats - 1) / feats * (((long long)n + rows - 1) / rows);
+    long long want = (rows < 64 ? 4 : 2) * (long long)sm_count();
+    int segments = simt_segments(k);
+    if (tiles >= want)
+        return 1;
+    return (int)((want + tiles - 1) / tiles < segments ? (want + tiles - 1) / tiles : segments);
+}
+
+template <typename TA, typename TW, typename Tile>
+static bool simt_launch(const void *A, const void *W, float *out, int n, int m, int k, int groups, bool vec,
+                        bool early, cudaStream_t st)
+{
+    static unsigned long long done = 0, done_parts = 0;
+    constexpr int smem = Tile::template smem<TA, TW>();
+    long long row_tiles = ((long long)n + Tile::ROWS - 1) / Tile::ROWS;
+    long long tiles = row_tiles * (((long long)m + Tile::FEATS - 1) / Tile::FEATS);
+    if (tiles > 0x7fffffffll)
+        return false;
+    dim3 grid((unsigned)tiles, 1, groups);
+    if (groups > 1) {
+        if (!allow_dynamic_smem(gemm_simt_kernel<TA, TW, Tile, true>, smem, done_parts))
+            return false;
+        launch(gemm_simt_kernel<TA, TW, Tile, true>, grid, Tile::THREADS, smem, st, (const TA *)A, (const TW *)W, out,
+               n, m, k, (int)row_tiles, vec, early);
+    } else {
+        if (!allow_dynamic_smem(gemm_simt_kernel<TA, TW, Tile, false>, smem, done))
+            return false;
+        launch(gemm_simt_kernel<TA, TW, Tile, false>, grid, Tile::THREADS, smem, st, (const TA *)A, (const TW *)W, out,
+               n, m, k, (int)row_tiles, vec, early);
+    }
+    return true;
+}
+
+template <typename TA, typename TW>
+static bool simt_pick(const void *A, const void *W, float *out, int n, int m, int k, int groups, bool early,
+                      cudaStream_t st)
+{
+    bool vec = ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0) && k % (16 / (int)sizeof(TA)) == 0 &&
+               k % (16 / (int)sizeof(TW)) == 0;
+    if (n <= 8)
+        return simt_launch<TA, TW, Rows8>(A, W, out, n, m, k, groups, vec, early, st);
+    if (n <= 16)
+        return simt_launch<TA, TW, Rows16>(A, W, out, n, m, k, groups, vec, early, st);
+    if (n <= 32)
+        return simt_launch<TA, TW, Rows32>(A, W, out, n, m, k, groups, vec, early, st);
+    return simt_launch<TA, TW, Rows64>(A, W, out, n, m, k, groups, vec, early, st);
 }
 
 }  // namespace jb
@@ -233,54 +351,47 @@ using namespace jb;
 // Floats of scratch that jb_gemm_simt wants for this shape (0: none).
 extern "C" long long jb_gemm_simt_scratch(int n, int m, int k)
 {
-    int segments = (k + SEG - 1) / SEG;
-    if (n <= 0 || n > SK_MAX_N || segments <= 1)
+    if (n <= 0 || m <= 0 || k <= 0 || simt_groups(n, m, k) <= 1)
         return 0;
-    return (long long)segments * n * m;
+    return (long long)simt_segments(k) * n * m;
 }
 
-// scratch: jb_gemm_simt_scratch(n, m, k) floats (may be null when that is 0).
+// scratch: jb_gemm_simt_scratch(n, m, k) floats (may be null when that is 0).  early: W was complete before
+// any kernel that may still run (a model's weights), so it may be read before the kernel ahead has ended.
 extern "C" int jb_gemm_simt(const void *A, int a_dt, const void *W, int w_dt, float *out, int n,
-                            int m, int k, float *scratch, cudaStream_t st)
+                            int m, int k, float *scratch, int early, cudaStream_t st)
 {
     if (n <= 0 || m <= 0)
         return JB_OK;
-    if (k <= 0)
+    if (k <= 0 || ((long long)n + 63) / 64 > 65535)
         return JB_EINVAL;
-    dim3 grid((m + BN - 1) / BN, (n + BM - 1) / BM);
-    if (grid.y > 65535)
+    int groups = simt_groups(n, m, k), segments = simt_segments(k);
+    if (groups > 1 && scratch == nullptr)
         return JB_EINVAL;
-    bool vec = k % 4 == 0 && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-    bool skinny = n <= SK_MAX_N;
-    int segments = (k + SEG - 1) / SEG;
-    if (skinny && segments > 1 && scratch == nullptr)
+    float *to = groups > 1 ? scratch : out;
+    bool ok;
+    if (a_dt == JB_F32 && w_dt == JB_F32)
+        ok = simt_pick<float, float>(A, W, to, n, m, k, groups, early != 0, st);
+    else if (a_dt == JB_F32 && w_dt == JB_BF16)
+        ok = simt_pick<float, bf16>(A, W, to, n, m, k, groups, early != 0, st);
+    else if (a_dt == JB_BF16 && w_dt == JB_F32)
+        ok = simt_pick<bf16, float>(A, W, to, n, m, k, groups, early != 0, st);
+    else if (a_dt == JB_BF16 && w_dt == JB_BF16)
+        ok = simt_pick<bf16, bf16>(A, W, to, n, m, k, groups, early != 0, st);
+    else
         return JB_EINVAL;
-    dim3 sgrid((m + SK_FEATS - 1) / SK_FEATS, segments);
-    float *part = segments > 1 ? scratch : out;
-#define JB_GEMM(TA, TW)                                                                       \
-    if (skinny)                                                                               \
-        launch(gemm_simt_skinny_kernel<TA, TW>, sgrid, SK_THREADS, 0, st, (const TA *)A,      \
-               (const TW *)W, part, n, m, k, vec);                                            \
-    else                                                                                      \
-        launch(gemm_simt_kernel<TA, TW>, grid, 256, 0, st, (const TA *)A, (const TW *)W, out, n, m, k, vec)
-    if (a_dt == JB_F32 && w_dt == JB_F32) {
-        JB_GEMM(float, float);
-    } else if (a_dt == JB_F32 && w_dt == JB_BF16) {
-        JB_GEMM(float, bf16);
-    } else if (a_dt == JB_BF16 && w_dt == JB_F32) {
-        JB_GEMM(bf16, float);
-    } else if (a_dt == JB_BF16 && w_dt == JB_BF16) {
-        JB_GEMM(bf16, bf16);
-    } else {
-        return JB_EINVAL;
-    }
-#undef JB_GEMM
-    if (skinny && segments > 1) {
+    if (!ok)
+        return JB_ELAUNCH;
+    if (groups > 1) {
         if (cudaGetLastError() != cudaSuccess)
             return JB_ELAUNCH;
         long long count = (long long)n * m;
-        launch(gemm_simt_join_kernel, (unsigned)((count + 255) / 256), 256, 0, st, (const float *)part,
-               out, count, segments);
+        if (count % 4 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)scratch % 16 == 0)
+            launch(gemm_simt_join_kernel<4>, (unsigned)((count / 4 + 255) / 256), 256, 0, st, (const float *)scratch,
+                   out, count, segments);
+        else
+            launch(gemm_simt_join_kernel<1>, (unsigned)((count + 255) / 256), 256, 0, st, (const float *)scratch, out,
+                   count, segments);
     }
     return launch_status();
 }

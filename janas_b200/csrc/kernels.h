@@ -304,7 +304,7 @@ int jb_attention_merge_gen(const float *scratch, const int32_t *row_pos, void *o
 int jb_attn_tc_error(void);
 long long jb_gemm_simt_scratch(int n, int m, int k);
 int jb_gemm_simt(const void *A, int a_dt, const void *W, int w_dt, float *out, int n, int m, int k,
-                 float *scratch, cudaStream_t st);
+                 float *scratch, int early, cudaStream_t st);
 int jb_gemm_tc_ok(const void *A, const void *W, int n, int m, int k);
 int jb_gemm_tc_splits(int n, int m, int k);
 int jb_gemm_tc(const void *A, const void *W, float *out, int n, int m, int k, int splits,

@@ -624,7 +624,7 @@ Stack linear(Device &d, const void *a, DType a_dt, long long n, long long k, con
     long long need = jb_gemm_simt_scratch(ni, mi, ki);
     Buf scratch;
     if (need > 0) scratch = d.pool.get((size_t)need * 4);
-    check(jb_gemm_simt(a, a_dt, w.ptr, w.dt, out.data(), ni, mi, ki, scratch.as<float>(), d.stream),
+    check(jb_gemm_simt(a, a_dt, w.ptr, w.dt, out.data(), ni, mi, ki, scratch.as<float>(), 1, d.stream),
           "linear", need > 0 ? 2 : 1);
     return out;
 }
@@ -657,7 +657,7 @@ HeadStack linear_heads(Device &d, const void *a, DType a_dt, int H, long long n,
     for (int h = 0; h < H && n > 0; h++) {
         const char *ah = (const char *)a + h * a_head, *wh = (const char *)w.ptr + h * w_head;
         float *oh = out.data() + (size_t)h * one;
-        check(jb_gemm_simt(ah, a_dt, wh, w.dt, oh, ni, mi, ki, scratch.as<float>(), d.stream),
+        check(jb_gemm_simt(ah, a_dt, wh, w.dt, oh, ni, mi, ki, scratch.as<float>(), 1, d.stream),
               "linear_heads", need > 0 ? 2 : 1);
     }
     return out;

@@ -1211,7 +1211,7 @@ def linear(a: torch.Tensor, weight: torch.Tensor, force_simt: bool = False,
     need = int(L.jb_gemm_simt_scratch(n, m, k))
     scratch = torch.empty((need,), dtype=torch.float32, device=a.device) if need else None
     _check(L.jb_gemm_simt(_p(a), _DT[a.dtype], _p(weight), _DT[weight.dtype], _p(out), n, m,
-                          k, _p(scratch), _stream()), "linear", kernels=2 if need else 1)
+                          k, _p(scratch), 0, _stream()), "linear", kernels=2 if need else 1)
     return out
 
 

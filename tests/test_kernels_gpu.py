@@ -110,6 +110,23 @@ def test_rmsnorm_many_rows(wdt, n, dm, S):
     assert ((got - want).abs().max(dim=1).values <= 2 ** -8 * want.abs().max(dim=1).values).all()
 
 
+@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32),
+                                     (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("m,k", [(64, 64), (65, 96), (129, 511), (200, 512), (63, 516), (130, 1544), (2560, 4100),
+                                 (20000, 520)])
+def test_gemm_simt_rows(adt, wdt, m, k):
+    """Every tile of rows (8, 16, 32, 64) at its edges: a row's bits do not depend on the rows beside it, and the
+    error is that of the recipe's chains: 256 products, the segments' sums, one rounding of the widest sum each."""
+    a, w = rnd(67, k, dtype=adt), rnd(m, k, dtype=wdt, seed=3)
+    a_dev, w_dev = a.to(DEV), w.to(DEV)
+    whole = ops().linear(a_dev, w_dev, force_simt=True)[0]
+    want = a.double() @ w.double().T
+    bound = (258 + k // 512) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert ((whole.cpu().double() - want).abs() <= bound).all()
+    for n in (1, 8, 9, 16, 17, 32, 33, 64, 65):
+        assert torch.equal(ops().linear(a_dev[:n].contiguous(), w_dev, force_simt=True)[0], whole[:n]), n
+
+
 @pytest.mark.parametrize("odt", DTYPES)
 def test_swiglu(odt):
     n, ff = 7, 300
