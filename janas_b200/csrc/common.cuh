@@ -121,6 +121,35 @@ __device__ __forceinline__ float gated_unit(float g, float u, const GatedUnit &p
     return g / (1.0f + expf(-p.alpha * g)) * (u + p.shift);
 }
 
+// Two floats side by side, and one multiply-add of both (each rounded like fmaf).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float sum2(f32x2 v)
+{
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 pair2(float lo, float hi)
+{
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void split2(f32x2 v, float &lo, float &hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
 // Programmatic dependent launch.  Every kernel of this library is launched with
 // the attribute that lets its CTAs start while the kernel before it in the
 // stream is still running.  pdl_trigger() (early in a kernel) allows the next

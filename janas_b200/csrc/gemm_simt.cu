@@ -28,19 +28,6 @@ static_assert(SEG % BK == 0, "segments end where stages end");
 // values a row of a stage takes in shared memory: a multiple of 16 bytes, and neighbouring rows start in other banks
 template <typename T> constexpr int ROW = BK + 16 / (int)sizeof(T);
 
-// Two floats side by side, and one multiply-add of both (each rounded like fmaf).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ float sum2(f32x2 v)
-{
-    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
-}
-
 // Four consecutive values of a row in shared memory as two pairs.
 __device__ __forceinline__ void pairs(const float *p, f32x2 &lo, f32x2 &hi)
 {
