@@ -4,10 +4,11 @@
 // A row (one token of one sequence, at position pos) sees the positions
 // lo..pos of its own sequence, lo = max(0, pos + 1 - window) with a window and
 // 0 without.  The positions are cut into chunks of ATT_CHUNK that start at
-// absolute positions; one warp computes, for one (row, KV head, chunk), the
+// absolute positions; a block computes, for one (row, KV head, chunk), the
 // partial softmax of every query head of the group: the largest score m, the
-// sum l of exp(score - m) and the values weighted by them.  A second kernel
-// merges a row's partials in chunk order.  Both steps depend only on the row's
+// sum l of exp(score - m) and the values weighted by them, a warp for every
+// quarter of the chunk, joined in order.  A second kernel merges a row's
+// partials in chunk order.  Both steps depend only on the row's
 // own position and keys, so a row's result is the same bits whether it runs in
 // a whole prompt, alone as a decoded token, or beside other sequences.
 //
@@ -81,7 +82,11 @@ __host__ __device__ inline size_t part_at(size_t row, int nh, int h, int max_chu
     return ((row * nh + h) * max_chunks + ci) * (size_t)(hd + 2);
 }
 
-// LPK lanes share one key (16 values of the head each); 32 / LPK keys a step.
+// LPK lanes share one key (16 values of the head each); 32 / LPK keys a step.  What bounds it is the chain of a
+// warp's steps: the next step's keys and values are asked for before this step's are used, and a warp has a
+// quarter of a chunk.  One B200, float, 32 heads on 8 of 128, microseconds for partials and merge (before: a warp
+// per chunk, each step's loads waited for): 8 rows at contexts of 32 to 1,024 62 -> 17, a prompt of 300 rows
+// 217 -> 192.
 template <typename T, int LPK>
 __global__ void __launch_bounds__(128)
 attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
@@ -94,12 +99,12 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
                     const float *__restrict__ score_bias)
 {
     constexpr int KPW = 32 / LPK;
+    constexpr int QUARTER = ATT_CHUNK / 4;
+    __shared__ float so[4][ATT_GT][LPK * 16], sml[4][ATT_GT][2];
     pdl_trigger();
     pdl_wait();
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    size_t item = (size_t)blockIdx.x * 4 + warp;
-    if (item >= (size_t)n_rows * max_chunks)
-        return;
+    size_t item = blockIdx.x;
     int lrow = (int)(item / max_chunks), ci = (int)(item % max_chunks);
     int row = row0 + lrow;
     int kvh = blockIdx.y;
@@ -126,6 +131,10 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
         t0 = max(lo, c * ATT_CHUNK);
         t1 = min(pos, c * ATT_CHUNK + ATT_CHUNK - 1);
     }
+
+    // this warp's quarter of the chunk
+    t0 = max(t0, c * ATT_CHUNK + warp * QUARTER);
+    t1 = min(t1, c * ATT_CHUNK + warp * QUARTER + QUARTER - 1);
 
     int cidx = lane % LPK, ks = lane / LPK;
     // a lane's 16 values of the keys (and q) and of the values; heads that are no
@@ -169,24 +178,39 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
     for (int g = 0; g < ATT_GT; g++)
         sb[g] = score_bias != nullptr && g < gt ? score_bias[h0 + g] : 0.0f;
 
+    // a step's key and value of this lane's key, zeros where there is none
+    float kn[16], vn[16];
+    auto ask = [&](int t) {
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+            kn[j] = vn[j] = 0.0f;
+        if (t > t1)
+            return;
+        size_t at = ((size_t)bt[t / PAGE] * nkv + kvh) * PAGE + (t % PAGE);
+        if (has_dims) {
+            if (vec_k)
+                load16<T>(k_cache + at * hd + cidx * 16, kn);
+            else
+                load_some<T>(k_cache + at * hd + cidx * 16, kn, cnt_k);
+        }
+        if (has_vals) {
+            if (vec_v)
+                load16<T>(v_cache + at * v_ld + cidx * 16, vn);
+            else
+                load_some<T>(v_cache + at * v_ld + cidx * 16, vn, cnt_v);
+        }
+    };
+    ask(t0 + ks);
     for (int base = t0; base <= t1; base += KPW) {
         int t = base + ks;
         bool valid = t <= t1;
-        float kv[16];
+        float kv[16], vv[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++)
-            kv[j] = 0.0f;
-        size_t at = 0;
-        if (valid) {
-            int page = bt[t / PAGE];
-            at = ((size_t)page * nkv + kvh) * PAGE + (t % PAGE);
-            if (has_dims) {
-                if (vec_k)
-                    load16<T>(k_cache + at * hd + cidx * 16, kv);
-                else
-                    load_some<T>(k_cache + at * hd + cidx * 16, kv, cnt_k);
-            }
+        for (int j = 0; j < 16; j++) {
+            kv[j] = kn[j];
+            vv[j] = vn[j];
         }
+        ask(t + KPW);
         float s[ATT_GT];
 #pragma unroll
         for (int g = 0; g < ATT_GT; g++) {
@@ -205,23 +229,13 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
             if (slopes != nullptr)
                 s[g] -= sl[g] * (float)(pos - t);
         }
-        if (valid && has_vals) {
-            if (vec_v)
-                load16<T>(v_cache + at * v_ld + cidx * 16, kv);
-            else
-                load_some<T>(v_cache + at * v_ld + cidx * 16, kv, cnt_v);
-        } else if (valid) {
-#pragma unroll
-            for (int j = 0; j < 16; j++)
-                kv[j] = 0.0f;
-        }
         if (valid && score_bias != nullptr) {
 #pragma unroll
             for (int g = 0; g < ATT_GT; g++) {
                 float p = 1.0f / (1.0f + expf(-(s[g] + sb[g])));
 #pragma unroll
                 for (int j = 0; j < 16; j++)
-                    o[g][j] = fmaf(p, kv[j], o[g][j]);
+                    o[g][j] = fmaf(p, vv[j], o[g][j]);
             }
         } else if (valid) {
 #pragma unroll
@@ -233,7 +247,7 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
                 l[g] = l[g] * a + p;
 #pragma unroll
                 for (int j = 0; j < 16; j++)
-                    o[g][j] = o[g][j] * a + p * kv[j];
+                    o[g][j] = o[g][j] * a + p * vv[j];
             }
         }
     }
@@ -260,23 +274,35 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
         }
     }
 
+    // the quarters into one, in order
     if (ks == 0) {
 #pragma unroll
         for (int g = 0; g < ATT_GT; g++) {
-            if (g >= gt)
-                continue;
-            float *dst = part + part_at((size_t)lrow, nh, h0 + g, max_chunks, ci, vd);
             if (lane == 0) {
-                dst[0] = m[g];
-                dst[1] = l[g];
+                sml[warp][g][0] = m[g];
+                sml[warp][g][1] = l[g];
             }
-            if (has_vals) {
 #pragma unroll
-                for (int j = 0; j < 16; j++)
-                    if (j < cnt_v)
-                        dst[2 + cidx * 16 + j] = o[g][j];
-            }
+            for (int j = 0; j < 16; j++)
+                so[warp][g][cidx * 16 + j] = o[g][j];
         }
+    }
+    __syncthreads();
+    for (int g = 0; g < gt; g++) {
+        float mn = fmaxf(fmaxf(sml[0][g][0], sml[1][g][0]), fmaxf(sml[2][g][0], sml[3][g][0]));
+        float f[4], sum = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            f[w] = score_bias != nullptr ? 1.0f : mn == -INFINITY ? 0.0f : expf(sml[w][g][0] - mn);
+            sum = fmaf(sml[w][g][1], f[w], sum);
+        }
+        float *dst = part + part_at((size_t)lrow, nh, h0 + g, max_chunks, ci, vd);
+        if (threadIdx.x == 0) {
+            dst[0] = mn;
+            dst[1] = sum;
+        }
+        for (int d = threadIdx.x; d < vd; d += 128)
+            dst[2 + d] = fmaf(so[3][g][d], f[3], fmaf(so[2][g][d], f[2], fmaf(so[1][g][d], f[1], so[0][g][d] * f[0])));
     }
 }
 
@@ -776,7 +802,9 @@ static int attention_typed(const T *q, const T *k_cache, const T *v_cache, const
         lpk <<= 1;
     int group = nh / nkv;
     size_t items = (size_t)n_rows * max_chunks;
-    dim3 grid((unsigned)((items + 3) / 4), nkv, (group + ATT_GT - 1) / ATT_GT);
+    if (items > 0x7fffffff)
+        return JB_EINVAL;
+    dim3 grid((unsigned)items, nkv, (group + ATT_GT - 1) / ATT_GT);
 #define JB_ATT(L)                                                                            \
     launch(attn_partial_kernel<T, L>, grid, 128, 0, st, q, k_cache, v_cache, row_pos, row_seq, \
            block_table, bt_stride, part, row0, n_rows, nh, nkv, hd, vd, window, scale,        \
