@@ -61,6 +61,14 @@ def _params(dtype, max_tokens: int, max_seqs: Optional[int], device, n_ctx: Opti
     return p
 
 
+def _ints(values: Sequence[int]):
+    """C int32 of a sequence whose members ``int`` takes."""
+    try:
+        return lib.i32_array(values)
+    except TypeError:
+        return lib.i32_array([int(v) for v in values])
+
+
 class PendingDecode:
     """A decode step under way: ``result()`` waits for it and gives its tokens."""
 
@@ -226,8 +234,8 @@ class Engine:
         for i, e in enumerate(entries):
             if not isinstance(e, StepEntry):
                 e = StepEntry(*e)
-            toks = lib.i32_array(int(t) for t in e.tokens)
-            want = lib.i32_array(int(w) for w in e.want)
+            toks = _ints(e.tokens)
+            want = _ints(e.want)
             keep += [toks, want]
             arr[i].slot = int(e.slot)
             arr[i].n = len(e.tokens)
@@ -295,8 +303,8 @@ class Engine:
         """Launches a decode step (one token for each slot, the next token chosen on
         the device) and returns at once; ``tokens=None``: the slots go on from the
         tokens the step begun last chose for them."""
-        sl = lib.i32_array(int(s) for s in slots)
-        tk = None if tokens is None else lib.i32_array(int(t) for t in tokens)
+        sl = _ints(slots)
+        tk = None if tokens is None else _ints(tokens)
         h = ctypes.c_void_p()
         code = lib.lib().jb_llm_decode_begin(self._h, sl, len(slots), tk, int(bool(sampled)),
                                              ctypes.byref(h))
