@@ -693,65 +693,6 @@ gated_part_norm_kernel(const float *y, const float *pre, int pre_S, size_t pre_s
     }
 }
 
-// The same for parts of up to NV values a thread: all of a thread's loads go out together and its values stay in
-// registers.  The sums run in the order of the kernel above.  2,048 rows of 2,560 values, one part and a sigmoid
-// after it, or eight parts and a silu ahead: 41 us before.
-template <typename TO, int NV>
-__global__ void __launch_bounds__(256)
-gated_part_norm_regs_kernel(const float *y, const float *pre, int pre_S, size_t pre_stride, int pre_ld, int pre_col0,
-                            const float *post, int post_S, size_t post_stride, int post_ld, int post_col0,
-                            const float *__restrict__ w, float eps, TO *__restrict__ out, int width, int parts,
-                            int post_silu, PartScale ps)
-{
-    __shared__ float red[32];
-    pdl_trigger();
-    int r = blockIdx.x, part = blockIdx.y, len = width / parts, c0 = part * len;
-    float *mp = part_maximum(ps, r, part);
-    pdl_wait();
-    float v[NV], g[NV], m_new = 0.0f;
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        int c = threadIdx.x + i * blockDim.x;
-        v[i] = c < len ? y[(size_t)r * width + c0 + c] : 0.0f;
-    }
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        int c = threadIdx.x + i * blockDim.x;
-        g[i] = pre != nullptr && c < len ? add_partials(0.0f, pre + (size_t)r * pre_ld + pre_col0 + c0 + c, pre_S, pre_stride) : 0.0f;
-    }
-    const float div = part_factor(ps, r, part, parts, mp, m_new);
-    float ss = 0.0f;
-#pragma unroll
-    for (int i = 0; i < NV; i++)
-        if (threadIdx.x + i * blockDim.x < len) {
-            v[i] *= div;
-            if (pre != nullptr)
-                v[i] *= silu_f(g[i]);
-            ss = fmaf(v[i], v[i], ss);
-        }
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        int c = threadIdx.x + i * blockDim.x;
-        g[i] = post != nullptr && c < len ? add_partials(0.0f, post + (size_t)r * post_ld + post_col0 + c0 + c, post_S, post_stride) : 0.0f;
-    }
-    ss = block_sum(ss, red);
-    if (mp != nullptr && threadIdx.x == 0)
-        *mp = m_new;           // every thread has read the old one: block_sum met them all
-    float scale = 1.0f / sqrtf(ss / (float)len + eps);
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        int c = threadIdx.x + i * blockDim.x;
-        if (c >= len)
-            break;
-        float o = v[i] * scale;
-        if (w != nullptr)
-            o *= w[c0 + c];
-        if (post != nullptr)
-            o *= post_silu ? silu_f(g[i]) : sigmoid_f(g[i]);
-        out[(size_t)r * width + c0 + c] = from_f<TO>(o);
-    }
-}
-
 // The same for short parts (a head's values each): a warp per (row, part), four neighbouring values
 // a lane and up to U of those; lengths, columns and rows are multiples of four.
 template <typename TO, int U>
@@ -988,46 +929,6 @@ pair_combine_kernel(const float *L, int SL, size_t strideL, const float *R, int 
             out[(size_t)r * m + c] = sl * ((u * fl) * wl[c]) + sr * ((v * fr) * wr[c]);
         else
             out[(size_t)r * m + c] = fmaf(fl, u, fr * v);
-    }
-}
-
-// The normed sum for rows of up to 256 NV values: both results are read once, all of a thread's loads together, and
-// stay in registers.  The sums run in the order of the kernel above.  2,048 rows of 2,560: 38 us before.
-template <int NV>
-__global__ void __launch_bounds__(256)
-pair_combine_regs_kernel(const float *L, int SL, size_t strideL, const float *R, int SR, size_t strideR,
-                         const float *__restrict__ wl, const float *__restrict__ wr, float sl, float sr, float eps,
-                         float *__restrict__ out, int m)
-{
-    __shared__ float red[32];
-    pdl_trigger();
-    int r = blockIdx.x;
-    pdl_wait();
-    float u[NV], v[NV], a = 0.0f, b = 0.0f;
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        int c = threadIdx.x + 256 * i;
-        u[i] = c < m ? add_partials(0.0f, L + (size_t)r * m + c, SL, strideL) : 0.0f;
-    }
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        int c = threadIdx.x + 256 * i;
-        v[i] = c < m ? add_partials(0.0f, R + (size_t)r * m + c, SR, strideR) : 0.0f;
-    }
-#pragma unroll
-    for (int i = 0; i < NV; i++)
-        if (threadIdx.x + 256 * i < m) {
-            a = fmaf(u[i], u[i], a);
-            b = fmaf(v[i], v[i], b);
-        }
-    a = block_sum(a, red);
-    b = block_sum(b, red);
-    float fl = 1.0f / sqrtf(a / (float)m + eps), fr = 1.0f / sqrtf(b / (float)m + eps);
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        int c = threadIdx.x + 256 * i;
-        if (c < m)
-            out[(size_t)r * m + c] = sl * ((u[i] * fl) * wl[c]) + sr * ((v[i] * fr) * wr[c]);
     }
 }
 
@@ -1358,20 +1259,6 @@ static int part_norm_launch(const float *y, const float *pre, int pre_S, long lo
     int keep = len * 4 <= 40 * 1024 ? 1 : 0;
     size_t smem = keep ? len * 4 : 0;
     int threads = len >= 1024 ? 256 : 128;
-    // parts that a block's registers hold
-    if (len <= (size_t)threads * 16 && (out_dt == JB_F32 || out_dt == JB_BF16)) {
-#define JB_GPR(TO, NV)                                                                                                 \
-    launch(gated_part_norm_regs_kernel<TO, NV>, grid, threads, 0, st, y, pre, pre_S, (size_t)pre_stride, pre_ld, pre_col0,   \
-           post, post_S, (size_t)post_stride, post_ld, post_col0, w, eps, (TO *)out, width, parts, post_silu, ps)
-        const bool four_each = len <= (size_t)threads * 4, twelve_each = len <= (size_t)threads * 12;
-        if (out_dt == JB_F32) {
-            if (four_each) JB_GPR(float, 4); else if (twelve_each) JB_GPR(float, 12); else JB_GPR(float, 16);
-        } else {
-            if (four_each) JB_GPR(bf16, 4); else if (twelve_each) JB_GPR(bf16, 12); else JB_GPR(bf16, 16);
-        }
-#undef JB_GPR
-        return launch_status();
-    }
     if (out_dt == JB_F32)
         launch(gated_part_norm_kernel<float>, grid, threads, smem, st, y, pre, pre_S, (size_t)pre_stride, pre_ld, pre_col0,
                post, post_S, (size_t)post_stride, post_ld, post_col0, w, eps, (float *)out, width, parts, keep, post_silu, ps);
@@ -1468,14 +1355,6 @@ extern "C" int jb_pair_combine(const float *L, int SL, long long strideL, const 
                            (size_t)strideL, R, SR, (size_t)strideR, wl, wr, sl, sr, eps, out, m, cols);
             return launch_status();
         }
-    }
-    if (wl != nullptr && m <= 4096) {
-#define JB_PCR(NV)                                                                                               \
-    launch(pair_combine_regs_kernel<NV>, (unsigned)n, 256, 0, st, L, SL, (size_t)strideL, R, SR, (size_t)strideR, wl, \
-           wr, sl, sr, eps, out, m)
-        if (m <= 1024) JB_PCR(4); else if (m <= 3072) JB_PCR(12); else JB_PCR(16);
-#undef JB_PCR
-        return launch_status();
     }
     launch(pair_combine_kernel, (unsigned)n, 256, 0, st, L, SL, (size_t)strideL, R, SR, (size_t)strideR, wl, wr, sl, sr,
            eps, out, m);

@@ -284,15 +284,6 @@ causal_conv_rows_kernel(const float *u, int ld, int col0, const float *__restric
         in_pos[q] = row_pos[rr];
         in_seq[q] = row_seq[rr];
     }
-    // the rows before the first, asked for with the others (whether they count is seen below)
-    float4 back[KEEP];
-    int back_seq[KEEP];
-#pragma unroll
-    for (int k = 1; k <= KEEP; k++) {
-        int rr = max(r0 - k, 0);
-        back[k - 1] = RB > 1 ? load4(in + (size_t)rr * ld) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        back_seq[k - 1] = RB > 1 && r0 - k >= 0 ? row_seq[rr] : -1;
-    }
 #pragma unroll
     for (int q = 0; q < RB; q++) {
         int r = r0 + q;
@@ -306,8 +297,6 @@ causal_conv_rows_kernel(const float *u, int ld, int col0, const float *__restric
                 int p = pos - k;
                 if (p < 0)
                     hist[k - 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                else if (q == 0 && RB > 1 && back_seq[k - 1] == seq)
-                    hist[k - 1] = plus(back[k - 1]);
                 else if (r - k >= 0 && row_seq[r - k] == seq)
                     hist[k - 1] = plus(load4(in + (size_t)(r - k) * ld));
                 else

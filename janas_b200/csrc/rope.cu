@@ -466,91 +466,81 @@ qkv_prepare_append_kernel(const float *__restrict__ qkv, int S, size_t split_str
 // 16-byte boundaries (8 for a bfloat16 cache): one load of four sums per lane, the sum of
 // squares over the slot's lanes, and the rotation's partner (rot_half values on, that is
 // rot_half / 4 lanes on) by a shuffle of the finished values.
-struct PrepareArgs {
-    const float *qkv;
-    int S;
-    size_t split_stride;
-    int ld;
-    const float *bias, *q_w, *k_w;
-    float eps;
-    const float *cs, *sn;
-    int rot_half;
-    const int32_t *row_pos, *row_seq, *block_table;
-    int bt_stride, n, nh, nkv, hd, vd, mode;
-};
-
-// what a lane (l of its slot's L) holds of a row's angles
-__device__ __forceinline__ void prepare_angles(const PrepareArgs &a, int pos, int l, float4 &co, float4 &si)
+template <typename TC, int L>
+__global__ void __launch_bounds__(128)
+qkv_prepare_append_vec_kernel(const float *__restrict__ qkv, int S, size_t split_stride, int ld,
+                              const float *__restrict__ bias, const float *__restrict__ q_w,
+                              const float *__restrict__ k_w, float eps, const float *__restrict__ cs,
+                              const float *__restrict__ sn, int rot_half,
+                              const int32_t *__restrict__ row_pos, const int32_t *__restrict__ row_seq,
+                              const int32_t *__restrict__ block_table, int bt_stride,
+                              TC *__restrict__ q_out, TC *__restrict__ k_cache, TC *__restrict__ v_cache,
+                              int n, int nh, int nkv, int hd, int vd, int mode)
 {
-    co = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    si = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (a.mode & JB_ROT_PAIRS) {
+    constexpr int PER_WARP = 32 / L;
+    const bool pairs = mode & JB_ROT_PAIRS, unit = mode & JB_UNIT_NORM, both = mode & JB_VALUES_FROM_KEYS;
+    pdl_trigger();
+    unsigned slots = nh + (both ? 1 : 2) * nkv;
+    unsigned total = (unsigned)n * slots;
+    unsigned task = (blockIdx.x * blockDim.y + threadIdx.y) * PER_WARP + threadIdx.x / L;
+    bool live = task < total;
+    if (!live)
+        task = total - 1;          // the lanes stay for the shuffles and store nothing
+    unsigned row = task / slots, hs = task - row * slots;
+    int l = threadIdx.x % L, group0 = threadIdx.x - l;
+    bool is_q = hs < (unsigned)nh;
+    bool is_v = hs >= (unsigned)(nh + nkv);
+    int pos = row_pos[row];
+    int page = k_cache != nullptr ? block_table[(size_t)row_seq[row] * bt_stride + pos / PAGE] : 0;
+    const float *w = is_v ? nullptr : is_q ? q_w : k_w;
+    int len = is_v ? vd : hd;
+    int hl = is_v ? 0 : rot_half / 4;                // lanes to a half of the rotated part
+    size_t col0 = is_q ? (size_t)hs * hd
+                       : !is_v ? (size_t)nh * hd + (size_t)(hs - nh) * hd
+                               : (size_t)(nh + nkv) * hd + (size_t)(hs - nh - nkv) * vd;
+    bool has = 4 * l < len;
+    float4 wv = make_float4(1.0f, 1.0f, 1.0f, 1.0f), co = wv, si = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (w != nullptr && has)
+        wv = load4(w + 4 * l);
+    if (pairs) {
         // a lane's four values are two pairs: angles 2 l and 2 l + 1 (in co.x, co.y)
-        if (2 * l < a.rot_half) {
-            const float2 c2 = *reinterpret_cast<const float2 *>(a.cs + (size_t)pos * a.rot_half + 2 * l);
-            const float2 s2 = *reinterpret_cast<const float2 *>(a.sn + (size_t)pos * a.rot_half + 2 * l);
+        if (!is_v && 2 * l < rot_half) {
+            const float2 c2 = *reinterpret_cast<const float2 *>(cs + (size_t)pos * rot_half + 2 * l);
+            const float2 s2 = *reinterpret_cast<const float2 *>(sn + (size_t)pos * rot_half + 2 * l);
             co.x = c2.x; co.y = c2.y; si.x = s2.x; si.y = s2.y;
         }
-    } else {
-        int hl = a.rot_half / 4;                     // lanes to a half of the rotated part
-        if (l < 2 * hl) {
-            int f = 4 * (l < hl ? l : l - hl);
-            co = load4(a.cs + (size_t)pos * a.rot_half + f);
-            si = load4(a.sn + (size_t)pos * a.rot_half + f);
-        }
+    } else if (l < 2 * hl) {
+        int f = 4 * (l < hl ? l : l - hl);
+        co = load4(cs + (size_t)pos * rot_half + f);
+        si = load4(sn + (size_t)pos * rot_half + f);
     }
-}
-
-// the slot's sums (the product's parts and the bias) in this lane
-__device__ __forceinline__ float4 prepare_load(const PrepareArgs &a, unsigned row, unsigned hs, int l)
-{
-    bool is_q = hs < (unsigned)a.nh, is_v = hs >= (unsigned)(a.nh + a.nkv);
-    size_t col0 = is_q ? (size_t)hs * a.hd
-                       : !is_v ? (size_t)a.nh * a.hd + (size_t)(hs - a.nh) * a.hd
-                               : (size_t)(a.nh + a.nkv) * a.hd + (size_t)(hs - a.nh - a.nkv) * a.vd;
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (4 * l < (is_v ? a.vd : a.hd)) {
-        const float *src = a.qkv + (size_t)row * a.ld + col0 + 4 * l;
-        if (a.bias != nullptr)
-            v = load4(a.bias + col0 + 4 * l);
-        for (int sp = 0; sp < a.S; sp++) {
-            float4 u = load4(src + (size_t)sp * a.split_stride);
-            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-        }
-    }
-    return v;
-}
-
-// norms, rotation and the store of one slot; every lane of the warp calls it.  wq, wk: the lane's weights.
-template <typename TC, int L>
-__device__ __forceinline__ void prepare_slot(const PrepareArgs &a, unsigned row, unsigned hs, bool live, int l, int pos,
-                                             int page, float4 v, const float4 &wq, const float4 &wk, const float4 &co,
-                                             const float4 &si, TC *__restrict__ q_out, TC *__restrict__ k_cache,
-                                             TC *__restrict__ v_cache)
-{
-    const bool pairs = a.mode & JB_ROT_PAIRS, unit = a.mode & JB_UNIT_NORM, both = a.mode & JB_VALUES_FROM_KEYS;
-    const int rot_half = a.rot_half;
-    bool is_q = hs < (unsigned)a.nh, is_v = hs >= (unsigned)(a.nh + a.nkv);
-    int group0 = threadIdx.x - l, len = is_v ? a.vd : a.hd;
-    int hl = is_v ? 0 : rot_half / 4;
-    bool has = 4 * l < len;
+    pdl_wait();
     TC *dst = nullptr;
     if (is_q) {
-        dst = q_out + ((size_t)row * a.nh + hs) * a.hd;
+        dst = q_out + ((size_t)row * nh + hs) * hd;
     } else if (k_cache != nullptr) {
-        int kvh = !is_v ? hs - a.nh : hs - a.nh - a.nkv;
-        size_t at = ((size_t)page * a.nkv + kvh) * PAGE + (pos % PAGE);
-        dst = !is_v ? k_cache + at * a.hd : v_cache + at * a.vd;
+        int kvh = !is_v ? hs - nh : hs - nh - nkv;
+        size_t at = ((size_t)page * nkv + kvh) * PAGE + (pos % PAGE);
+        dst = !is_v ? k_cache + at * hd : v_cache + at * vd;
     }
-    if (has && both && !is_q && live && dst != nullptr)
-        store4(v_cache + (dst - k_cache) + 4 * l, v);      // vd = hd: the same place in the value pages
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (has) {
+        const float *src = qkv + (size_t)row * ld + col0 + 4 * l;
+        if (bias != nullptr)
+            v = load4(bias + col0 + 4 * l);
+        for (int sp = 0; sp < S; sp++) {
+            float4 u = load4(src + (size_t)sp * split_stride);
+            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+        }
+        if (both && !is_q && live && dst != nullptr)
+            store4(v_cache + (dst - k_cache) + 4 * l, v);      // vd = hd: the same place in the value pages
+    }
     float ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1)
         ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (!is_v && a.q_w != nullptr) {
-        const float4 wv = is_q ? wq : wk;
-        float scale = 1.0f / sqrtf(ss / (float)len + a.eps);
+    if (w != nullptr) {
+        float scale = 1.0f / sqrtf(ss / (float)len + eps);
         v.x = (v.x * scale) * wv.x; v.y = (v.y * scale) * wv.y;
         v.z = (v.z * scale) * wv.z; v.w = (v.w * scale) * wv.w;
     }
@@ -580,75 +570,12 @@ __device__ __forceinline__ void prepare_slot(const PrepareArgs &a, unsigned row,
         for (int o = L / 2; o > 0; o >>= 1)
             s2 += __shfl_xor_sync(0xffffffffu, s2, o);
         if (!is_v) {
-            float after = 1.0f / sqrtf(s2 / (float)len + a.eps);
+            float after = 1.0f / sqrtf(s2 / (float)len + eps);
             v.x *= after; v.y *= after; v.z *= after; v.w *= after;
         }
     }
     if (live && has && dst != nullptr)
         store4(dst + 4 * l, v);
-}
-
-// Few rows: a warp per 32 / L slots.
-template <typename TC, int L>
-__global__ void __launch_bounds__(128)
-qkv_prepare_append_vec_kernel(const PrepareArgs a, TC *__restrict__ q_out, TC *__restrict__ k_cache, TC *__restrict__ v_cache)
-{
-    constexpr int PER_WARP = 32 / L;
-    pdl_trigger();
-    unsigned slots = a.nh + ((a.mode & JB_VALUES_FROM_KEYS) ? 1 : 2) * a.nkv;
-    unsigned total = (unsigned)a.n * slots;
-    unsigned task = (blockIdx.x * blockDim.y + threadIdx.y) * PER_WARP + threadIdx.x / L;
-    bool live = task < total;
-    if (!live)
-        task = total - 1;          // the lanes stay for the shuffles and store nothing
-    unsigned row = task / slots, hs = task - row * slots;
-    int l = threadIdx.x % L;
-    int pos = a.row_pos[row];
-    int page = k_cache != nullptr ? a.block_table[(size_t)a.row_seq[row] * a.bt_stride + pos / PAGE] : 0;
-    float4 w = make_float4(1.0f, 1.0f, 1.0f, 1.0f), co, si;
-    if (a.q_w != nullptr && hs < (unsigned)(a.nh + a.nkv) && 4 * l < a.hd)
-        w = load4((hs < (unsigned)a.nh ? a.q_w : a.k_w) + 4 * l);
-    prepare_angles(a, pos, l, co, si);
-    pdl_wait();
-    prepare_slot<TC, L>(a, row, hs, live, l, pos, page, prepare_load(a, row, hs, l), w, w, co, si, q_out, k_cache, v_cache);
-}
-
-// Many rows: a block per row, whose warps share the row's slots out.  A row's place, angles and weights are then
-// found once, and four slots' sums are on their way together; with a warp per slot (above) those and the
-// addresses were two of three of its 300 instructions.  2,048 rows of 48 slots of 128 (76 MB), beside the
-// layer's other kernels: 41 us before.
-template <typename TC, int L>
-__global__ void __launch_bounds__(128)
-qkv_prepare_append_many_kernel(const PrepareArgs a, TC *__restrict__ q_out, TC *__restrict__ k_cache, TC *__restrict__ v_cache)
-{
-    constexpr int PER_WARP = 32 / L, PER_PASS = 4 * PER_WARP;
-    pdl_trigger();
-    const int slots = a.nh + ((a.mode & JB_VALUES_FROM_KEYS) ? 1 : 2) * a.nkv;
-    const unsigned row = blockIdx.x;
-    const int l = threadIdx.x % L, first = threadIdx.y * PER_WARP + threadIdx.x / L;
-    int pos = a.row_pos[row];
-    int page = k_cache != nullptr ? a.block_table[(size_t)a.row_seq[row] * a.bt_stride + pos / PAGE] : 0;
-    float4 wq = make_float4(1.0f, 1.0f, 1.0f, 1.0f), wk = wq, co, si;
-    if (a.q_w != nullptr && 4 * l < a.hd) {
-        wq = load4(a.q_w + 4 * l);
-        wk = load4(a.k_w + 4 * l);
-    }
-    prepare_angles(a, pos, l, co, si);
-    pdl_wait();
-    for (int p0 = 0; p0 < slots; p0 += 4 * PER_PASS) {
-        float4 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-            v[u] = prepare_load(a, row, (unsigned)min(p0 + u * PER_PASS + first, slots - 1), l);
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            if (p0 + u * PER_PASS >= slots)
-                break;                     // the same for the whole block
-            int hs = p0 + u * PER_PASS + first;
-            prepare_slot<TC, L>(a, row, (unsigned)min(hs, slots - 1), hs < slots, l, pos, page, v[u], wq, wk, co, si, q_out,
-                                k_cache, v_cache);
-        }
-    }
 }
 
 }  // namespace jb
@@ -687,19 +614,10 @@ extern "C" int jb_qkv_prepare_append(const float *qkv, int S, long long split_st
         int L = big <= 32 ? 8 : big <= 64 ? 16 : 32;
         size_t warps = (tasks + (32 / L) - 1) / (32 / L);
         unsigned g = (unsigned)((warps + 3) / 4);
-        const PrepareArgs args{qkv, S, (size_t)split_stride, ld, bias, q_w, k_w, eps, cs, sn, rot_half, row_pos, row_seq,
-                               block_table, bt_stride, n, nh, nkv, hd, vd, mode};
-        // (a block for every place on the chip: below that a warp per slot finishes sooner)
-        const bool many = n >= 8 * sm_count() && nh + nkv > 0;
 #define JB_QPV(TC, LL)                                                                                  \
-    do {                                                                                                \
-        if (many)                                                                                       \
-            launch(qkv_prepare_append_many_kernel<TC, LL>, (unsigned)n, block, 0, st, args, (TC *)q_out, \
-                   (TC *)k_cache, (TC *)v_cache);                                                       \
-        else                                                                                            \
-            launch(qkv_prepare_append_vec_kernel<TC, LL>, g, block, 0, st, args, (TC *)q_out,           \
-                   (TC *)k_cache, (TC *)v_cache);                                                       \
-    } while (0)
+    launch(qkv_prepare_append_vec_kernel<TC, LL>, g, block, 0, st, qkv, S, (size_t)split_stride, ld, bias, \
+           q_w, k_w, eps, cs, sn, rot_half, row_pos, row_seq, block_table, bt_stride, (TC *)q_out,       \
+           (TC *)k_cache, (TC *)v_cache, n, nh, nkv, hd, vd, mode)
 #define JB_QPV_L(TC)                                                                                    \
     do {                                                                                                \
         if (L == 8) JB_QPV(TC, 8);                                                                      \

@@ -268,44 +268,6 @@ def test_a_sequences_bits_do_not_depend_on_the_batch(kind):
         assert torch.equal(alone[1], both[1])
 
 
-@pytest.mark.parametrize("hd,vd,nh,nkv,rot,mode", [(128, 128, 5, 2, 32, "pairs"), (64, 48, 7, 1, 16, "unit"),
-                                                   (32, 32, 3, 3, 8, "both"), (128, 128, 13, 4, 0, "")])
-def test_prepared_rows_keep_their_bits_among_many(hd, vd, nh, nkv, rot, mode):
-    """1,300 rows go a block a row, 100 of them alone a warp a head: the same queries, keys and values."""
-    n, flags = 1300, dict(pairs=mode == "pairs", unit_norm=mode == "unit", values_from_keys=mode == "both")
-    width = nh * hd + nkv * hd + (0 if mode == "both" else nkv * vd)
-    qkv = rnd(2, n, width + 4, seed=1).to(DEV)
-    pos = torch.arange(n, dtype=torch.int32, device=DEV)
-    table = torch.arange((n + 63) // 64, dtype=torch.int32, device=DEV).flip(0).contiguous()[None]
-    cos, sin = (torch.cos(rnd(n, rot, seed=2)).to(DEV), torch.sin(rnd(n, rot, seed=2)).to(DEV)) if rot else (None, None)
-    qw, kw = (1 + 0.2 * rnd(hd, seed=s).to(DEV) for s in (3, 4))
-    for dtype in (torch.float32, torch.bfloat16):
-        def run(lo, hi, caches):
-            seq = torch.zeros(hi - lo, dtype=torch.int32, device=DEV)
-            return ops().qkv_prepare_append(qkv[:, lo:hi].contiguous(), None, qw, kw, 1e-5, cos, sin, pos[lo:hi].contiguous(),
-                                            seq, table, caches[0], caches[1], nh, **flags)
-        one, few = ([torch.zeros(table.shape[1], nkv, 64, d, dtype=dtype, device=DEV) for d in (hd, vd)] for _ in range(2))
-        whole = run(0, n, one)
-        parts = torch.cat([run(i, i + 100, few) for i in range(0, n, 100)])
-        assert torch.equal(whole, parts) and all(torch.equal(a, b) for a, b in zip(one, few))
-
-
-@pytest.mark.parametrize("width,parts", [(512, 1), (516, 1), (1540, 1), (3072, 1), (3076, 1), (4096, 1), (4100, 1), (2600, 8)])
-def test_norms_of_rows_held_in_registers(width, parts):
-    """Row and part lengths on both sides of what a thread's registers hold: 4, 12 and 16 values."""
-    n = 3
-    y, g, z = rnd(n, width, seed=1), rnd(1, n, width + 8, seed=2), rnd(2, n, width, seed=3)
-    w, w2 = 1 + 0.1 * rnd(width, seed=4), 1 + 0.1 * rnd(width, seed=5)
-    v = (y.double() * pm.silu(g[0, :, 4:4 + width].double())).view(n, parts, -1)
-    rms = lambda x: x / torch.sqrt((x * x).mean(dim=-1, keepdim=True) + 1e-5)          # noqa: E731
-    got = ops().gated_part_norm(y.to(DEV), parts, w.to(DEV), 1e-5, torch.float32, pre=g.to(DEV), pre_col0=4,
-                                post=z.to(DEV)).cpu()
-    close(got, (rms(v).reshape(n, width) * w * torch.sigmoid(z.double().sum(0))).float(), 3e-6)
-    L, R = z.double().sum(0), g[0, :, :width].double()
-    got = ops().pair_combine(z.to(DEV), g[:, :, :width].contiguous().to(DEV), w.to(DEV), w2.to(DEV), 0.5, 0.7, 1e-5).cpu()
-    close(got, (0.5 * rms(L) * w + 0.7 * rms(R) * w2).float(), 3e-6)
-
-
 def test_a_key_far_back_in_the_state():
     """A decay of exactly 1 keeps a key for good, a decay of 0.9 loses it: one key is written 700 tokens
     before the query that asks for it, among keys that are orthogonal to it."""
