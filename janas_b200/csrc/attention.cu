@@ -29,43 +29,40 @@ namespace jb {
 constexpr int ATT_CHUNK = 128;  // positions per partial (two pages)
 constexpr int ATT_GT = 4;       // query heads a warp carries at once
 
-template <typename T> __device__ __forceinline__ void load16(const T *p, float *out);
-
-template <> __device__ __forceinline__ void load16<float>(const float *p, float *out)
+// The 16 values of a head that lane c of LPK holds lie in groups of 16 bytes (4 floats, 8 bfloat16), LPK groups
+// apart, so that the lanes of a key read its row in whole lines.  Place of value j; the load of all 16 from a row
+// p of `count` values, zeros beyond it (vec: the row's length is a multiple of a group, every row on 16 bytes).
+template <typename T, int LPK> __device__ __forceinline__ int lane_value(int c, int j)
 {
-    const float4 *q = reinterpret_cast<const float4 *>(p);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        float4 v = q[i];
-        out[4 * i + 0] = v.x;
-        out[4 * i + 1] = v.y;
-        out[4 * i + 2] = v.z;
-        out[4 * i + 3] = v.w;
-    }
+    constexpr int GS = 16 / sizeof(T);
+    return (j / GS * LPK + c) * GS + j % GS;
 }
 
-template <> __device__ __forceinline__ void load16<bf16>(const bf16 *p, float *out)
+template <typename T, int LPK>
+__device__ __forceinline__ void load16(const T *p, float *out, int c, int count, bool vec)
 {
-    const uint4 *q = reinterpret_cast<const uint4 *>(p);
+    constexpr int GS = 16 / sizeof(T);
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-        uint4 v = q[i];
-        uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    for (int g = 0; g < 16 / GS; g++) {
+        int d = (g * LPK + c) * GS;
+        if (vec) {
+            uint4 v = d < count ? *reinterpret_cast<const uint4 *>(p + d) : make_uint4(0, 0, 0, 0);
+            uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            out[8 * i + 2 * j + 0] = __uint_as_float(w[j] << 16);
-            out[8 * i + 2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+            for (int j = 0; j < 4; j++) {
+                if constexpr (GS == 4) {
+                    out[4 * g + j] = __uint_as_float(w[j]);
+                } else {
+                    out[8 * g + 2 * j] = __uint_as_float(w[j] << 16);
+                    out[8 * g + 2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < GS; j++)
+                out[GS * g + j] = d + j < count ? to_f(p[d + j]) : 0.0f;
         }
     }
-}
-
-// Up to 16 values of a head whose size is no multiple of 16 (rows of such heads
-// lie at no 16-byte boundary): one by one, zeros beyond `count`.
-template <typename T> __device__ __forceinline__ void load_some(const T *p, float *out, int count)
-{
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-        out[j] = j < count ? to_f(p[j]) : 0.0f;
 }
 
 // Partials that the kept first tokens of a windowed mixer take: their chunks.
@@ -83,8 +80,8 @@ __host__ __device__ inline size_t part_at(size_t row, int nh, int h, int max_chu
 }
 
 // LPK lanes share one key (16 values of the head each); 32 / LPK keys a step.  What bounds it is the chain of a
-// warp's steps: the next step's keys and values are asked for before this step's are used, and a warp has a
-// quarter of a chunk.  One B200, float, 32 heads on 8 of 128, microseconds for partials and merge (before: a warp
+// warp's steps and, with every place taken, the lines that its loads touch: the next step's keys and values are
+// asked for before this step's are used, a warp has a quarter of a chunk, and a load takes whole lines.  One B200, float, 32 heads on 8 of 128, microseconds for partials and merge (before: a warp
 // per chunk, each step's loads waited for): 8 rows at contexts of 32 to 1,024 62 -> 17, a prompt of 300 rows
 // 217 -> 192.
 template <typename T, int LPK>
@@ -137,11 +134,9 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
     t1 = min(t1, c * ATT_CHUNK + warp * QUARTER + QUARTER - 1);
 
     int cidx = lane % LPK, ks = lane / LPK;
-    // a lane's 16 values of the keys (and q) and of the values; heads that are no
-    // multiple of 16 are read value by value
-    bool has_dims = cidx * 16 < hd, has_vals = cidx * 16 < vd;
-    bool vec_k = hd % 16 == 0, vec_v = vd % 16 == 0 && v_ld % 16 == 0;
-    int cnt_k = min(16, hd - cidx * 16), cnt_v = min(16, vd - cidx * 16);
+    constexpr int GS = 16 / sizeof(T);
+    const bool vec_k = hd % GS == 0 && (((uintptr_t)q | (uintptr_t)k_cache) & 15) == 0;
+    const bool vec_v = vd % GS == 0 && v_ld % GS == 0 && ((uintptr_t)v_cache & 15) == 0;
     const int32_t *bt = block_table + (size_t)row_seq[row] * bt_stride;
 
     float qv[ATT_GT][16], o[ATT_GT][16], m[ATT_GT], l[ATT_GT];
@@ -152,13 +147,8 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
 #pragma unroll
         for (int j = 0; j < 16; j++)
             o[g][j] = qv[g][j] = 0.0f;
-        if (g < gt && has_dims) {
-            const T *qp = q + ((size_t)row * nh + h0 + g) * hd + cidx * 16;
-            if (vec_k)
-                load16<T>(qp, qv[g]);
-            else
-                load_some<T>(qp, qv[g], cnt_k);
-        }
+        if (g < gt)
+            load16<T, LPK>(q + ((size_t)row * nh + h0 + g) * hd, qv[g], cidx, hd, vec_k);
     }
     // a head's own factor on its scores (1 when the mixer has none)
     float hs[ATT_GT];
@@ -187,18 +177,8 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
         if (t > t1)
             return;
         size_t at = ((size_t)bt[t / PAGE] * nkv + kvh) * PAGE + (t % PAGE);
-        if (has_dims) {
-            if (vec_k)
-                load16<T>(k_cache + at * hd + cidx * 16, kn);
-            else
-                load_some<T>(k_cache + at * hd + cidx * 16, kn, cnt_k);
-        }
-        if (has_vals) {
-            if (vec_v)
-                load16<T>(v_cache + at * v_ld + cidx * 16, vn);
-            else
-                load_some<T>(v_cache + at * v_ld + cidx * 16, vn, cnt_v);
-        }
+        load16<T, LPK>(k_cache + at * hd, kn, cidx, hd, vec_k);
+        load16<T, LPK>(v_cache + at * v_ld, vn, cidx, vd, vec_v);
     };
     ask(t0 + ks);
     for (int base = t0; base <= t1; base += KPW) {
@@ -284,7 +264,7 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
             }
 #pragma unroll
             for (int j = 0; j < 16; j++)
-                so[warp][g][cidx * 16 + j] = o[g][j];
+                so[warp][g][lane_value<T, LPK>(cidx, j)] = o[g][j];
         }
     }
     __syncthreads();

@@ -260,3 +260,32 @@ def test_steps_fed_on_the_device_equal_steps_fed_by_the_host(dtype):
     assert runs["device", False] == runs["host", False]
     assert runs["device", True] == runs["host", True]
     assert runs["host", True] != runs["host", False]
+
+
+def test_uneven_sequences_in_a_wide_decode_step():
+    """40 sequences on 8 KV heads are more pairs than the attention has places, and most are far shorter than the
+    longest: runs of nine chunks.  The step's logits are those of the sequences decoded alone (bfloat16), and the
+    captured step chooses their largest."""
+    from janas_b200.engine import Engine
+    cfg = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", num_hidden_layers=1, hidden_size=256,
+               num_attention_heads=16, num_key_value_heads=8, head_dim=128, intermediate_size=256, vocab_size=300,
+               rope_theta=1e6, rms_norm_eps=1e-6, tie_word_embeddings=False, max_position_embeddings=4096)
+    rng = np.random.default_rng(5)
+    lens = [1300, 1152, 1153, 2305] + [int(v) for v in rng.integers(1, 400, 36)]
+    prompts = [rng.integers(0, 300, n).tolist() for n in lens]
+    eng = Engine.open_random(cfg, 3, "bfloat16", max_tokens=sum(lens) + 64 * 80, max_seqs=40)
+    slots = [eng.new_sequence() for _ in lens]
+    for i in range(0, 40, 8):
+        eng.step([(s, p, []) for s, p in zip(slots[i:i + 8], prompts[i:i + 8])])
+    fed = rng.integers(0, 300, 40).tolist()
+    together = eng.step_numpy([(s, [t], [0]) for s, t in zip(slots, fed)])
+    for s, n in zip(slots, lens):
+        assert eng.truncate_sequence(s, n)
+    alone = np.concatenate([eng.step_numpy([(s, [t], [0])]) for s, t in zip(slots, fed)])
+    # one attention's weights and one result rounded to bfloat16, from sums of another order
+    assert np.abs(together - alone).max() <= 2 ** -6 * np.abs(alone).max()
+    for s, n in zip(slots, lens):
+        assert eng.truncate_sequence(s, n)
+    chosen = eng.decode(slots, fed)
+    assert (chosen == together.argmax(axis=1)).all()
+    eng.close()
