@@ -80,10 +80,12 @@ __host__ __device__ inline size_t part_at(size_t row, int nh, int h, int max_chu
 }
 
 // LPK lanes share one key (16 values of the head each); 32 / LPK keys a step.  What bounds it is the chain of a
-// warp's steps and, with every place taken, the lines that its loads touch: the next step's keys and values are
-// asked for before this step's are used, a warp has a quarter of a chunk, and a load takes whole lines.  One B200, float, 32 heads on 8 of 128, microseconds for partials and merge (before: a warp
-// per chunk, each step's loads waited for): 8 rows at contexts of 32 to 1,024 62 -> 17, a prompt of 300 rows
-// 217 -> 192.
+// warp's steps and, with every place taken, the instructions of each: a warp has a quarter of a chunk, loads run
+// a pair of steps ahead and take whole lines, and the weights are made once all scores are there, a lane a key,
+// instead of a rescaling of the sums at every key.  One B200, float, 32 heads on 8 of 128, microseconds (before:
+// a warp per chunk, key by key, each step's loads waited for): 8 rows at context 2,048 52 -> 41; two layers of a
+// prompt of 300 rows with their products 5,750 -> 3,708, of which the products' share is 1,800; 36 layers of a
+// prompt of 2,048 rows 636 -> 460 ms.
 template <typename T, int LPK>
 __global__ void __launch_bounds__(128)
 attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
@@ -97,7 +99,8 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
 {
     constexpr int KPW = 32 / LPK;
     constexpr int QUARTER = ATT_CHUNK / 4;
-    __shared__ float so[4][ATT_GT][LPK * 16], sml[4][ATT_GT][2];
+    static_assert(QUARTER == 32 && PAGE % QUARTER == 0, "a lane for every key of a quarter, all of one page");
+    __shared__ float so[4][ATT_GT][LPK * 16], sml[4][ATT_GT][2], sc[4][ATT_GT][QUARTER];
     pdl_trigger();
     pdl_wait();
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -139,120 +142,124 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
     const bool vec_v = vd % GS == 0 && v_ld % GS == 0 && ((uintptr_t)v_cache & 15) == 0;
     const int32_t *bt = block_table + (size_t)row_seq[row] * bt_stride;
 
-    float qv[ATT_GT][16], o[ATT_GT][16], m[ATT_GT], l[ATT_GT];
-#pragma unroll
-    for (int g = 0; g < ATT_GT; g++) {
-        m[g] = -INFINITY;
-        l[g] = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; j++)
-            o[g][j] = qv[g][j] = 0.0f;
-        if (g < gt)
-            load16<T, LPK>(q + ((size_t)row * nh + h0 + g) * hd, qv[g], cidx, hd, vec_k);
-    }
-    // a head's own factor on its scores (1 when the mixer has none)
-    float hs[ATT_GT];
-#pragma unroll
-    for (int g = 0; g < ATT_GT; g++)
-        hs[g] = head_scale != nullptr && g < gt ? head_scale[h0 + g] : 1.0f;
-    // a head's slope: slope * distance is taken off the score of a key that far back
-    float sl[ATT_GT];
-#pragma unroll
-    for (int g = 0; g < ATT_GT; g++)
-        sl[g] = slopes != nullptr && g < gt ? slopes[h0 + g] : 0.0f;
-    float inv_cap = softcap > 0.0f ? 1.0f / softcap : 0.0f;
-    // a number per head added to the score, whose sigmoid is then the key's weight:
-    // no maximum, no sum of weights
-    float sb[ATT_GT];
-#pragma unroll
-    for (int g = 0; g < ATT_GT; g++)
-        sb[g] = score_bias != nullptr && g < gt ? score_bias[h0 + g] : 0.0f;
-
-    // a step's key and value of this lane's key, zeros where there is none
-    float kn[16], vn[16];
-    auto ask = [&](int t) {
-#pragma unroll
-        for (int j = 0; j < 16; j++)
-            kn[j] = vn[j] = 0.0f;
-        if (t > t1)
-            return;
-        size_t at = ((size_t)bt[t / PAGE] * nkv + kvh) * PAGE + (t % PAGE);
-        load16<T, LPK>(k_cache + at * hd, kn, cidx, hd, vec_k);
-        load16<T, LPK>(v_cache + at * v_ld, vn, cidx, vd, vec_v);
-    };
-    ask(t0 + ks);
-    for (int base = t0; base <= t1; base += KPW) {
-        int t = base + ks;
-        bool valid = t <= t1;
-        float kv[16], vv[16];
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-            kv[j] = kn[j];
-            vv[j] = vn[j];
-        }
-        ask(t + KPW);
-        float s[ATT_GT];
-#pragma unroll
-        for (int g = 0; g < ATT_GT; g++) {
-            float d = 0.0f;
+    // The warp's 32 keys in three passes: their scores (LPK lanes a key, a pair of steps' keys on their way
+    // together) into shared memory; a lane a key for the largest, the weights and their sum; the values.
+    // Every key has its place by its position, so the sums' order is the row's own.
+    const int base = c * ATT_CHUNK + warp * QUARTER;
+    constexpr int U = LPK > 1 ? 2 : 1;
+    const size_t at0 = t0 <= t1 ? ((size_t)bt[base / PAGE] * nkv + kvh) * PAGE + base % PAGE : 0;   // (a quarter lies in one page)
+    auto seen = [&](int key) { return base + key >= t0 && base + key <= t1; };
+    auto ask = [&](const T *rows, int ld, int count, bool vec, int key, float (&x)[16]) {
+        if (seen(key)) {
+            load16<T, LPK>(rows + (at0 + key) * ld, x, cidx, count, vec);
+        } else {
 #pragma unroll
             for (int j = 0; j < 16; j++)
-                d = fmaf(qv[g][j], kv[j], d);
-#pragma unroll
-            for (int off = 1; off < LPK; off <<= 1)
-                d += __shfl_xor_sync(0xffffffffu, d, off);
-            s[g] = d * scale;
-            if (head_scale != nullptr)
-                s[g] *= hs[g];
-            if (softcap > 0.0f)
-                s[g] = softcap * tanhf(s[g] * inv_cap);
-            if (slopes != nullptr)
-                s[g] -= sl[g] * (float)(pos - t);
+                x[j] = 0.0f;
         }
-        if (valid && score_bias != nullptr) {
-#pragma unroll
-            for (int g = 0; g < ATT_GT; g++) {
-                float p = 1.0f / (1.0f + expf(-(s[g] + sb[g])));
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                    o[g][j] = fmaf(p, vv[j], o[g][j]);
-            }
-        } else if (valid) {
-#pragma unroll
-            for (int g = 0; g < ATT_GT; g++) {
-                float mn = fmaxf(m[g], s[g]);
-                float a = expf(m[g] - mn);  // 0 the first time (m = -inf)
-                float p = expf(s[g] - mn);
-                m[g] = mn;
-                l[g] = l[g] * a + p;
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                    o[g][j] = o[g][j] * a + p * vv[j];
-            }
-        }
-    }
-
-    // the 32 / LPK key groups of the warp into one
-#pragma unroll
-    for (int off = LPK; off < 32; off <<= 1) {
+    };
+    if (t0 <= t1) {
+        float qv[ATT_GT][16];
 #pragma unroll
         for (int g = 0; g < ATT_GT; g++) {
-            float mo = __shfl_xor_sync(0xffffffffu, m[g], off);
-            float lo_ = __shfl_xor_sync(0xffffffffu, l[g], off);
-            float mn = fmaxf(m[g], mo);
-            float a = mn == -INFINITY ? 0.0f : expf(m[g] - mn);
-            float b = mn == -INFINITY ? 0.0f : expf(mo - mn);
-            if (score_bias != nullptr)
-                a = b = 1.0f;           // plain sums
-            l[g] = l[g] * a + lo_ * b;
-            m[g] = mn;
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-                float oo = __shfl_xor_sync(0xffffffffu, o[g][j], off);
-                o[g][j] = o[g][j] * a + oo * b;
-            }
+            for (int j = 0; j < 16; j++)
+                qv[g][j] = 0.0f;
+            if (g < gt)
+                load16<T, LPK>(q + ((size_t)row * nh + h0 + g) * hd, qv[g], cidx, hd, vec_k);
+        }
+#pragma unroll 1
+        for (int st = 0; st < LPK; st += U) {
+            float kv[U][16];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                ask(k_cache, hd, hd, vec_k, (st + u) * KPW + ks, kv[u]);
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int g = 0; g < ATT_GT; g++) {
+                    float d = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        d = fmaf(qv[g][j], kv[u][j], d);
+#pragma unroll
+                    for (int off = 1; off < LPK; off <<= 1)
+                        d += __shfl_xor_sync(0xffffffffu, d, off);
+                    if (cidx == 0)
+                        sc[warp][g][(st + u) * KPW + ks] = d;
+                }
         }
     }
+    float vv[U][16];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        ask(v_cache, v_ld, vd, vec_v, u * KPW + ks, vv[u]);
+    __syncwarp();
+    float o[ATT_GT][16], m[ATT_GT], l[ATT_GT];
+    const float inv_cap = softcap > 0.0f ? 1.0f / softcap : 0.0f;
+#pragma unroll
+    for (int g = 0; g < ATT_GT; g++) {
+        bool on = g < gt && seen(lane);
+        float x = -INFINITY;
+        if (on) {
+            x = sc[warp][g][lane] * scale;
+            if (head_scale != nullptr)          // a head's own factor on its scores
+                x *= head_scale[h0 + g];
+            if (softcap > 0.0f)
+                x = softcap * tanhf(x * inv_cap);
+            if (slopes != nullptr)              // slope * distance is taken off the score of a key that far back
+                x -= slopes[h0 + g] * (float)(pos - (base + lane));
+        }
+        float p;
+        if (score_bias != nullptr) {
+            // the sigmoid of the score and a number per head is the key's weight: no maximum, no sum of weights
+            m[g] = -INFINITY;
+            l[g] = 0.0f;
+            p = on ? 1.0f / (1.0f + expf(-(x + score_bias[h0 + g]))) : 0.0f;
+        } else {
+            m[g] = warp_max(x);
+            p = on && m[g] != -INFINITY ? expf(x - m[g]) : 0.0f;
+            l[g] = warp_sum(p);
+        }
+        sc[warp][g][lane] = p;
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+            o[g][j] = 0.0f;
+    }
+    __syncwarp();
+    if (t0 <= t1) {
+#pragma unroll 1
+        for (int st = 0; st < LPK; st += U) {
+            float now[U][16];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    now[u][j] = vv[u][j];
+            if (st + U < LPK) {
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    ask(v_cache, v_ld, vd, vec_v, (st + U + u) * KPW + ks, vv[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int g = 0; g < ATT_GT; g++) {
+                    float p = sc[warp][g][(st + u) * KPW + ks];
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        o[g][j] = fmaf(p, now[u][j], o[g][j]);
+                }
+        }
+    }
+    // the 32 / LPK key groups of the warp into one
+#pragma unroll
+    for (int off = LPK; off < 32; off <<= 1)
+#pragma unroll
+        for (int g = 0; g < ATT_GT; g++)
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+                o[g][j] += __shfl_xor_sync(0xffffffffu, o[g][j], off);
 
     // the quarters into one, in order
     if (ks == 0) {
