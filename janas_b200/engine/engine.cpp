@@ -380,7 +380,8 @@ PendingDecode *Engine::decode_begin(const std::vector<int> &slots, const int32_t
     // positions keeps them close to what the step needs
     long long need = *std::max_element(p.pos0.begin(), p.pos0.end()) + 1;
     long long bound = std::min((need + 255) / 256 * 256, max_positions);
-    const bool rough = uneven(p.pos0);
+    // (a run of steps from the device's own tokens stays with what its first step was)
+    const bool rough = last_uneven_ = tokens ? uneven(p.pos0) : last_uneven_;
     GraphKey key((int)slots.size(), bound, sampled, long_way, rough);
     DecodeGraph *g = nullptr;
     for (auto it = graphs_.begin(); it != graphs_.end(); ++it) {

@@ -161,6 +161,7 @@ private:
     std::list<std::pair<GraphKey, std::unique_ptr<DecodeGraph>>> graphs_;
     DecodeGraph *last_graph_ = nullptr;     // the graph of the decode step begun last
     std::vector<int> last_slots_;
+    bool last_uneven_ = false;      // that step took its sequences for uneven
     std::vector<int> cache_entry_;          // run-order entry -> entry whose cache it uses, or -1
     std::unique_ptr<SamplerScratch> sampler_scratch_;
     PendingDecode eager_pending_;
