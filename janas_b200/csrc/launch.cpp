@@ -722,22 +722,10 @@ Buf attention_blocks(Device &d, const long long *row0, const long long *pos0, co
     return out;
 }
 
-static const int UNEVEN_CHUNKS = 9, ATTENTION_CHUNK = 128;
 // Into how many CTAs the chunks of one (token, KV head) pair are cut.  A CTA costs
 // about three chunks' time to set up, and CTAs beyond the device's places (two per
 // SM) come in waves: the cut that finishes first by that estimate.
-//
-// That takes every sequence for as long as the longest.  Where the pairs alone fill the places and
-// the sequences are uneven, the estimate leaves the longest ones' single CTAs running by themselves at
-// the end: a CTA then takes UNEVEN_CHUNKS chunks.  Three layers at 4B sizes, 64 sequences, microseconds a
-// step: lengths spread evenly over the logarithm up to 2,000 390 -> 367, up to 4,000 507 -> 440; spread
-// evenly up to 2,000 442 -> 424, up to 4,000 611 -> 563; all of 2,000 513 -> 531 (so not there).
-bool decode_uneven(long long pairs, long long sum, long long rows, long long longest, int places) {
-    return pairs > places && longest > (long long)UNEVEN_CHUNKS * ATTENTION_CHUNK && 4 * sum <= 3 * rows * longest;
-}
-
-static int decode_parts(long long pairs, int chunks, int places, bool uneven = false) {
-    if (uneven && pairs > places && chunks > UNEVEN_CHUNKS) return (chunks + UNEVEN_CHUNKS - 1) / UNEVEN_CHUNKS;
+static int decode_parts(long long pairs, int chunks, int places) {
     int best = 1;
     double best_t = -1;
     for (int parts = 1; parts <= chunks; parts++) {
@@ -786,7 +774,7 @@ Buf attention(Device &d, const void *q, long long n, const AttnCache &c, const A
         int win = std::max(max_chunks - kc, 1);
         parts = win;
         if (jb_attn_tc_decode_runs(g.nh, g.nkv, g.hd))
-            parts = decode_parts(std::min<long long>(n, 4096) * g.nkv, win, 2 * d.sm_count, c.uneven && !g.window);
+            parts = decode_parts(std::min<long long>(n, 4096) * g.nkv, win, 2 * d.sm_count);
         per_cta = (win + parts - 1) / parts;
         parts = kc + (win + per_cta - 1) / per_cta;
     }
@@ -831,7 +819,7 @@ Buf attention_decode_qkv(Device &d, const Stack &qkv, const DevTensor *q_w, cons
     }
     long long n = qkv.n;
     int ni = as_int(n, "rows");
-    int parts = decode_parts(std::min<long long>(n, 4096) * g.nkv, max_chunks, 2 * d.sm_count, c.uneven && !g.window);
+    int parts = decode_parts(std::min<long long>(n, 4096) * g.nkv, max_chunks, 2 * d.sm_count);
     int per_cta = (max_chunks + parts - 1) / parts;
     parts = (max_chunks + per_cta - 1) / per_cta;
     long long per_row = jb_attention_scratch(1, g.nh, g.hd, parts);

@@ -302,7 +302,6 @@ struct AttnCache {
     int bt_stride = 0;
     bool writes = true;
     int v_ld = 0;                          // the length of v's rows where it is not the values' head size
-    bool uneven = false;                   // a decode step whose sequences are mostly much shorter than the longest
 };
 
 // Per-head RMSNorm of q and k (when weights are given), NeoX rotation by the rows'
@@ -384,11 +383,6 @@ bool attention_prefill_ok(int nh, int nkv, int hd, int vd);
 Buf attention(Device &d, const void *q, long long n, const AttnCache &c, const AttnGeometry &g,
               const int32_t *row_pos, const int32_t *row_seq, int max_chunks, const int32_t *blocks,
               int n_blocks, bool decode, bool force_simt = false, bool head_major = false);
-
-// Whether a decode step's attention takes its sequences for uneven (AttnCache::uneven): pairs of (row, KV
-// head) beyond the device's places (two a SM), and lengths that add up to three quarters of `rows` times
-// the longest at most.
-bool decode_uneven(long long pairs, long long sum, long long rows, long long longest, int places);
 
 // qk_norm_rope_append and attention(decode) in one kernel, from the q,k,v product's
 // partial sums; an empty Buf where the kernel does not take these sizes and types.

@@ -145,18 +145,8 @@ Engine::Plan Engine::plan(const std::vector<StepEntry> &entries) const {
     return p;
 }
 
-bool Engine::uneven(const std::vector<long long> &pos0) const {
-    long long heads = 0, sum = 0, longest = 0;
-    for (auto &g : cache->groups) heads = std::max(heads, (long long)g->spec.num_kv_heads);
-    for (long long p : pos0) {
-        sum += p + 1;
-        longest = std::max(longest, p + 1);
-    }
-    return ops::decode_uneven((long long)pos0.size() * heads, sum, (long long)pos0.size(), longest, 2 * dev->sm_count);
-}
-
 std::vector<LayerCache> Engine::layer_caches(
-    const std::map<const KVGroup *, std::pair<const int32_t *, int>> &bt, bool uneven) {
+    const std::map<const KVGroup *, std::pair<const int32_t *, int>> &bt) {
     std::vector<LayerCache> out;
     for (size_t e = 0; e < model->spec.run_order.size(); e++) {
         LayerCache lc;
@@ -179,7 +169,6 @@ std::vector<LayerCache> Engine::layer_caches(
             lc.kv.v = g->v_of(src);
             lc.kv.n_pages = g->pool.n_pages();
             lc.kv.dt = cache->dtype;
-            lc.kv.uneven = uneven;
             auto it = bt.find(g);
             lc.kv.block_table = it->second.first;
             lc.kv.bt_stride = it->second.second;
@@ -264,7 +253,7 @@ Buf Engine::step(const std::vector<StepEntry> &entries, long long *n_wanted) {
     std::map<const KVGroup *, std::pair<const int32_t *, int>> bt;
     for (size_t gi = 0; gi < cache->groups.size(); gi++)
         bt[cache->groups[gi].get()] = {d + tab_off[gi], widths[gi]};
-    std::vector<LayerCache> caches = layer_caches(bt, p.kind == DECODE && uneven(p.pos0));
+    std::vector<LayerCache> caches = layer_caches(bt);
     Buf logits = model->forward(ctx, d, caches, all_rows ? nullptr : d + 3 * n + B, all_rows ? -1 : p.n_want);
     cache->advance(p.slots, p.lens);
     if (n_wanted) *n_wanted = p.n_want;
@@ -380,9 +369,7 @@ PendingDecode *Engine::decode_begin(const std::vector<int> &slots, const int32_t
     // positions keeps them close to what the step needs
     long long need = *std::max_element(p.pos0.begin(), p.pos0.end()) + 1;
     long long bound = std::min((need + 255) / 256 * 256, max_positions);
-    // (a run of steps from the device's own tokens stays with what its first step was)
-    const bool rough = last_uneven_ = tokens ? uneven(p.pos0) : last_uneven_;
-    GraphKey key((int)slots.size(), bound, sampled, long_way, rough);
+    GraphKey key((int)slots.size(), bound, sampled, long_way);
     DecodeGraph *g = nullptr;
     for (auto it = graphs_.begin(); it != graphs_.end(); ++it) {
         if (it->first == key) {
@@ -403,7 +390,7 @@ PendingDecode *Engine::decode_begin(const std::vector<int> &slots, const int32_t
             graphs_.pop_front();
         }
         graphs_.emplace_back(key, std::unique_ptr<DecodeGraph>(
-                                      new DecodeGraph(*this, (int)slots.size(), bound, sampled, long_way, rough)));
+                                      new DecodeGraph(*this, (int)slots.size(), bound, sampled, long_way)));
         g = graphs_.back().second.get();
     }
     DecodeGraph *before = tokens ? nullptr : last_graph_;

@@ -151,17 +151,13 @@ public:
 
 private:
     friend class DecodeGraph;
-    std::vector<LayerCache> layer_caches(const std::map<const KVGroup *, std::pair<const int32_t *, int>> &bt,
-                                         bool uneven);
-    // whether a decode step of sequences of these lengths is one of uneven sequences
-    bool uneven(const std::vector<long long> &pos0) const;
+    std::vector<LayerCache> layer_caches(const std::map<const KVGroup *, std::pair<const int32_t *, int>> &bt);
     // captured decode steps by (batch, context bound, sampled, long way); the one
     // used last at the back, the oldest goes when there are more than max_graphs
-    using GraphKey = std::tuple<int, long long, bool, bool, bool>;
+    using GraphKey = std::tuple<int, long long, bool, bool>;
     std::list<std::pair<GraphKey, std::unique_ptr<DecodeGraph>>> graphs_;
     DecodeGraph *last_graph_ = nullptr;     // the graph of the decode step begun last
     std::vector<int> last_slots_;
-    bool last_uneven_ = false;      // that step took its sequences for uneven
     std::vector<int> cache_entry_;          // run-order entry -> entry whose cache it uses, or -1
     std::unique_ptr<SamplerScratch> sampler_scratch_;
     PendingDecode eager_pending_;

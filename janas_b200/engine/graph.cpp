@@ -4,8 +4,8 @@
 
 namespace jb {
 
-DecodeGraph::DecodeGraph(Engine &e, int batch, long long bound, bool sampled, bool long_way, bool uneven)
-    : eng_(e), batch_(batch), bound_(bound), sampled_(sampled), long_way_(long_way), uneven_(uneven) {
+DecodeGraph::DecodeGraph(Engine &e, int batch, long long bound, bool sampled, bool long_way)
+    : eng_(e), batch_(batch), bound_(bound), sampled_(sampled), long_way_(long_way) {
     width_ = (int)((pages_for(bound) + 7) / 8 * 8);
     size_t n_groups = e.cache->groups.size();
     total_ = 4 * (size_t)batch + n_groups * (size_t)batch * (size_t)width_;
@@ -47,7 +47,7 @@ void DecodeGraph::launch(bool capturing) {
     std::map<const KVGroup *, std::pair<const int32_t *, int>> bt;
     for (size_t gi = 0; gi < e.cache->groups.size(); gi++)
         bt[e.cache->groups[gi].get()] = {d + 4 * (size_t)B + gi * (size_t)B * (size_t)width_, width_};
-    std::vector<LayerCache> caches = e.layer_caches(bt, uneven_);
+    std::vector<LayerCache> caches = e.layer_caches(bt);
     Buf logits = e.model->forward(ctx, d, caches, nullptr, -1);
     // the chosen tokens take the place of the tokens the step was fed
     ops::SamplerArrays s;

@@ -23,7 +23,7 @@ namespace jb {
 
 class DecodeGraph {
 public:
-    DecodeGraph(Engine &engine, int batch, long long bound, bool sampled, bool long_way, bool uneven);
+    DecodeGraph(Engine &engine, int batch, long long bound, bool sampled, bool long_way);
     ~DecodeGraph();
     DecodeGraph(const DecodeGraph &) = delete;
     DecodeGraph &operator=(const DecodeGraph &) = delete;
@@ -41,7 +41,7 @@ private:
     Engine &eng_;
     int batch_;
     long long bound_;
-    bool sampled_, long_way_, uneven_;
+    bool sampled_, long_way_;
     int width_;
     size_t total_;                      // int32 values of the input buffer
     int32_t *host_[2] = {nullptr, nullptr};

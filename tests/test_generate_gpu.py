@@ -264,8 +264,8 @@ def test_steps_fed_on_the_device_equal_steps_fed_by_the_host(dtype):
 
 def test_uneven_sequences_in_a_wide_decode_step():
     """40 sequences on 8 KV heads are more pairs than the attention has places, and most are far shorter than the
-    longest: runs of nine chunks.  The step's logits are those of the sequences decoded alone (bfloat16), and the
-    captured step chooses their largest."""
+    longest.  The step's logits are those of the sequences decoded alone (bfloat16), and the captured step chooses
+    their largest."""
     from janas_b200.engine import Engine
     cfg = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", num_hidden_layers=1, hidden_size=256,
                num_attention_heads=16, num_key_value_heads=8, head_dim=128, intermediate_size=256, vocab_size=300,
@@ -289,3 +289,56 @@ def test_uneven_sequences_in_a_wide_decode_step():
     chosen = eng.decode(slots, fed)
     assert (chosen == together.argmax(axis=1)).all()
     eng.close()
+
+
+WIDE = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", num_hidden_layers=2, hidden_size=256,
+            num_attention_heads=16, num_key_value_heads=8, head_dim=128, intermediate_size=256, vocab_size=300,
+            rope_theta=1e6, rms_norm_eps=1e-6, tie_word_embeddings=False, max_position_embeddings=4096)
+
+
+def wide_engine(lens, room=80):
+    """64 sequences of these lengths on 8 KV heads: more pairs than the decode attention has places."""
+    from janas_b200.engine import Engine
+    rng = np.random.default_rng(6)
+    eng = Engine.open_random(WIDE, 3, "bfloat16", max_tokens=sum(lens) + len(lens) * room, max_seqs=len(lens))
+    slots = [eng.new_sequence() for _ in lens]
+    prompts = [rng.integers(0, 300, 2400).tolist()[:n] for n in lens]     # a sequence's tokens whatever its length
+    eng.step([(slots[0], prompts[0], [])])          # (alone: a product's order of sums depends on the rows beside it)
+    for i in range(1, len(lens), 9):
+        eng.step([(s, p, []) for s, p in zip(slots[i:i + 9], prompts[i:i + 9])])
+    return eng, slots, rng.integers(0, 300, len(lens)).tolist()
+
+
+@pytest.mark.parametrize("longest", [1153, 1300, 2305])
+def test_a_wide_decode_step_keeps_a_sequence_whatever_the_others_lengths(longest):
+    """The longest sequence's logits are the same bits beside sequences as long as itself and beside short ones."""
+    rows = []
+    for others in (longest, 40):
+        eng, slots, fed = wide_engine([longest] + [others] * 63)
+        rows.append(eng.step_numpy([(s, [t], [0]) for s, t in zip(slots, fed)])[0])
+        eng.close()
+    assert (rows[0] == rows[1]).all()
+
+
+def test_wide_steps_fed_on_the_device_equal_steps_fed_by_the_host():
+    """As with few sequences: here on more pairs than the attention has places, uneven lengths, the longest going
+    past nine chunks of positions on the way.  Beside the tokens, the logits of one more step are compared: they
+    read the second layer's keys and values, which the first layer's attention went into."""
+    got = {}
+    for way in ("host", "device"):
+        eng, slots, toks = wide_engine([1148] + [30 + i for i in range(63)])
+        chosen = []
+        if way == "host":
+            for _ in range(8):
+                toks = eng.decode(slots, toks).tolist()
+                chosen.append(toks)
+        else:
+            cur = eng.decode_begin(slots, toks)
+            for i in range(8):
+                nxt = eng.decode_begin(slots, None) if i < 7 else None
+                chosen.append(eng.decode_end(cur).tolist())
+                cur = nxt
+        got[way] = chosen, eng.step_numpy([(s, [t], [0]) for s, t in zip(slots, chosen[-1])])
+        eng.close()
+    assert got["host"][0] == got["device"][0]
+    assert (got["host"][1] == got["device"][1]).all()
