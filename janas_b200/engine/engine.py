@@ -62,7 +62,9 @@ def _params(dtype, max_tokens: int, max_seqs: Optional[int], device, n_ctx: Opti
 
 
 def _ints(values: Sequence[int]):
-    """C int32 of a sequence whose members ``int`` takes."""
+    """C int32 of values that ``int`` takes."""
+    if not isinstance(values, (list, tuple)):
+        values = list(values)           # an iterator gives its values once
     try:
         return lib.i32_array(values)
     except TypeError:
@@ -304,7 +306,12 @@ class Engine:
         the device) and returns at once; ``tokens=None``: the slots go on from the
         tokens the step begun last chose for them."""
         sl = _ints(slots)
-        tk = None if tokens is None else _ints(tokens)
+        tk = None
+        if tokens is not None:
+            tokens = tokens if isinstance(tokens, (list, tuple)) else list(tokens)
+            if len(tokens) < len(slots):            # (as many are read)
+                raise StepError("decode: %d tokens for %d sequences" % (len(tokens), len(slots)))
+            tk = _ints(tokens)
         h = ctypes.c_void_p()
         code = lib.lib().jb_llm_decode_begin(self._h, sl, len(slots), tk, int(bool(sampled)),
                                              ctypes.byref(h))

@@ -1,0 +1,34 @@
+"""Tokens and slots as a caller may hand them to a step: any kind of whole number, in any kind of iterable."""
+from fractions import Fraction
+
+import numpy as np
+import pytest
+import torch
+
+from janas_b200.engine import Engine
+from janas_b200.engine.engine import StepError, _ints
+
+VALUES = [7, 0, -3, 2 ** 31 - 1]
+
+
+@pytest.mark.parametrize("kind", [int, float, str, np.int64, np.int32, np.float64, Fraction, torch.tensor])
+@pytest.mark.parametrize("hold", [list, tuple, iter, lambda v: (x for x in v), lambda v: dict.fromkeys(v).keys()])
+def test_packing(kind, hold):
+    assert list(_ints(hold([kind(v) for v in VALUES]))) == VALUES
+
+
+@pytest.mark.parametrize("values", [np.array(VALUES), np.array(VALUES, dtype=np.float64), torch.tensor(VALUES), range(5)])
+def test_packing_of_arrays(values):
+    assert list(_ints(values)) == [int(v) for v in values]
+
+
+def test_packing_of_nothing_leaves_a_place():
+    for none in ([], (), iter([]), np.array([], dtype=np.int32)):
+        assert list(_ints(none)) == [0]
+
+
+@pytest.mark.parametrize("tokens", [[], [5], (5,), iter([5]), iter([5.0]), np.array([5])])
+def test_a_decode_step_wants_a_token_for_every_slot(tokens):
+    eng = object.__new__(Engine)            # refused before the library is called
+    with pytest.raises(StepError, match="tokens for 2 sequences"):
+        eng.decode_begin([0, 1], tokens)
