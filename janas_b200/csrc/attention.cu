@@ -217,8 +217,8 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
             l[g] = 0.0f;
             p = on ? 1.0f / (1.0f + expf(-(x + score_bias[h0 + g]))) : 0.0f;
         } else {
-            m[g] = warp_max(x);
-            p = on && m[g] != -INFINITY ? expf(x - m[g]) : 0.0f;
+            m[g] = warp_max(x);         // (passes over NaN: a NaN score makes its own weight, and so the sums, NaN)
+            p = on && x != -INFINITY ? expf(x - m[g]) : 0.0f;
             l[g] = warp_sum(p);
         }
         sc[warp][g][lane] = p;

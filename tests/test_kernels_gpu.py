@@ -237,6 +237,31 @@ def test_attention_finds_a_far_key_and_the_window_s_edge(dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("what", [math.nan, math.inf, -math.inf])
+@pytest.mark.parametrize("nh,nkv,hd,window", [(6, 2, 32, 0), (4, 4, 16, 1), (8, 1, 80, 33), (5, 5, 80, 1), (2, 1, 320, 0)])
+def test_attention_keeps_what_is_not_finite(dtype, what, nh, nkv, hd, window):
+    """A key whose scores are NaN or infinite, alone in what a row sees or beside others: the row is what the softmax
+    in 64 bits makes of it (NaN beside NaN or +inf, nothing of a key of -inf, NaN where -inf is all there is)."""
+    n, chunk = 300, ops().attention_chunk()
+    q, k, v = rnd(n, nh, hd, dtype=dtype).abs() + 0.5, rnd(n, nkv, hd, dtype=dtype, seed=1), rnd(n, nkv, hd, dtype=dtype, seed=2)
+    mc = (n - 1) // chunk + 1 if not window else (window - 1) // chunk + 2
+    row, key = torch.arange(n)[:, None], torch.arange(n)[None]
+    seen = (key <= row) & (key > row - window if window else key >= 0)
+    for t in (0, 31, 32, 77, 128, 224, 299):
+        kt = k.clone()
+        kt[t, :, 0] = what
+        s = torch.einsum("nhd,mhd->hnm", q.double(), kt.double().repeat_interleave(nh // nkv, 1)) / math.sqrt(hd)
+        p = torch.where(seen, s, -math.inf).softmax(-1)
+        want = torch.einsum("hnm,mhd->nhd", p, v.double().repeat_interleave(nh // nkv, 1))
+        kc, vc, bt = paged(kt, v, 9)
+        got = ops().attention(q.to(DEV), kc.to(DEV), vc.to(DEV), row[:, 0].int().to(DEV), torch.zeros(n, dtype=torch.int32).to(DEV),
+                              bt.to(DEV), window, 1 / math.sqrt(hd), mc, force_simt=True).cpu().double()
+        assert torch.equal(got.isnan(), want.isnan()), t
+        tol = 5e-6 if dtype == torch.float32 else 2 ** -8
+        assert ((got - want).nan_to_num().abs() <= tol * want.nan_to_num().abs().max()).all(), t
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n0,n1,hd,nh,nkv", [(25, 15, 48, 6, 2), (300, 58, 128, 6, 2), (3, 1, 16, 6, 2),
                                              (40, 9, 32, 5, 1), (17, 30, 64, 9, 3),
                                              (9, 11, 256, 3, 3), (6, 3, 80, 4, 2),
