@@ -42,32 +42,66 @@ __device__ __forceinline__ void pairs(const bf16 *p, f32x2 &lo, f32x2 &hi)
     hi = (f32x2)(u.y & 0xffff0000u) << 32 | u.y << 16;
 }
 
-// Asks for ROWS rows of BK values from k0 on, src[row0 + r][k0 ..], to be put into a stage.
-// Rows from `have` on and values from kb on become zeros.  vec: 16 bytes at a time, asynchronously.
-template <typename T, int ROWS, int THREADS>
-__device__ __forceinline__ void fetch(T *stage, const T *__restrict__ src, long long row0, int have, int k,
-                                      int k0, int kb, bool vec)
+// Asks for ROWS rows of BK values from k0 on, src[row0 + r][k0 ..], to be put into a stage, BYTES (4, 8 or 16) at a
+// time; 2 bytes: values loaded and stored, sixteen of a thread on their way together.  Rows from `have` on and values
+// from kb on become zeros; k and kb are multiples of what a copy takes.
+template <typename T, int ROWS, int THREADS, int BYTES>
+__device__ __forceinline__ void fetch_by(T *stage, const T *__restrict__ src, long long row0, int have, int k,
+                                         int k0, int kb)
 {
-    constexpr int V = 16 / sizeof(T), PER = BK / V;
-    if (vec) {
+    constexpr int V = BYTES / sizeof(T), PER = BK / V, STEP = THREADS / PER, N = ROWS / STEP;
+    static_assert(THREADS % PER == 0 && ROWS % STEP == 0, "a thread has the same place in every STEP-th row");
+    int r = threadIdx.x / PER, c = threadIdx.x % PER * V;
+    const T *p = src + (row0 + r) * (size_t)k + k0 + c;
+    int rows = k0 + c < kb ? (int)min(have - row0, (long long)ROWS) - r : 0;
+    T *dst = stage + r * ROW<T> + c;
+    if constexpr (BYTES == 2) {
+        constexpr int B = N < 16 ? N : 16;
+#pragma unroll 1
+        for (int i = 0; i < N; i += B) {
+            T v[B];
 #pragma unroll
-        for (int i0 = 0; i0 < ROWS * PER; i0 += THREADS) {
-            int i = i0 + threadIdx.x;
-            if (ROWS * PER % THREADS && i >= ROWS * PER)
-                break;
-            int r = i / PER, c = (i % PER) * V;
-            bool in = row0 + r < have && k0 + c < kb;
-            const T *p = in ? src + (row0 + r) * (size_t)k + k0 + c : src;
-            uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + r * ROW<T> + c);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(p), "r"(in ? 16 : 0)
-                         : "memory");
+            for (int u = 0; u < B; u++) {
+                v[u] = (i + u) * STEP < rows ? *p : from_f<T>(0.0f);
+                p += STEP * (size_t)k;
+            }
+#pragma unroll
+            for (int u = 0; u < B; u++)
+                dst[(i + u) * STEP * ROW<T>] = v[u];
         }
     } else {
-        for (int i = threadIdx.x; i < ROWS * BK; i += THREADS) {
-            int r = i / BK, c = i % BK;
-            stage[r * ROW<T> + c] = row0 + r < have && k0 + c < kb ? src[(row0 + r) * (size_t)k + k0 + c] : from_f<T>(0.0f);
+        constexpr int UNROLL = BYTES == 16 || N < 8 ? N : 8;
+        uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+#pragma unroll UNROLL
+        for (int i = 0; i < N; i++) {
+            bool in = i * STEP < rows;
+            const T *from = in ? p : src;
+            if constexpr (BYTES == 16)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(in ? 16 : 0)
+                             : "memory");
+            else
+                asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(to), "l"(from), "n"(BYTES),
+                             "r"(in ? BYTES : 0)
+                             : "memory");
+            p += STEP * (size_t)k;
+            to += STEP * ROW<T> * (int)sizeof(T);
         }
     }
+}
+
+// bytes: what copy_bytes said.
+template <typename T, int ROWS, int THREADS>
+__device__ __forceinline__ void fetch(T *stage, const T *__restrict__ src, long long row0, int have, int k,
+                                      int k0, int kb, int bytes)
+{
+    if (bytes == 16)
+        fetch_by<T, ROWS, THREADS, 16>(stage, src, row0, have, k, k0, kb);
+    else if (bytes == 8)
+        fetch_by<T, ROWS, THREADS, 8>(stage, src, row0, have, k, k0, kb);
+    else if (sizeof(T) == 4 || bytes == 4)
+        fetch_by<T, ROWS, THREADS, 4>(stage, src, row0, have, k, k0, kb);
+    else if constexpr (sizeof(T) == 2)
+        fetch_by<T, ROWS, THREADS, 2>(stage, src, row0, have, k, k0, kb);
 }
 
 // A block's threads stand TX along the features and TY along the rows; a thread owns the rows
@@ -91,7 +125,7 @@ template <int RT, int CT, int TX, int TY, int ST> struct SimtTile {
 template <typename TA, typename TW, typename Tile, bool PARTS>
 __global__ void __launch_bounds__(Tile::THREADS, Tile::ROWS == 64 ? 2 : 1)
 gemm_simt_kernel(const TA *A, const TW *__restrict__ W, float *__restrict__ out, int n, int m, int k, int row_tiles,
-                 bool vec, bool early)
+                 int a_bytes, int w_bytes, bool early)
 {
     constexpr int RT = Tile::R, CT = Tile::C, TX = Tile::X, TY = Tile::Y, ST = Tile::STAGES, THREADS = Tile::THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -119,21 +153,21 @@ gemm_simt_kernel(const TA *A, const TW *__restrict__ W, float *__restrict__ out,
     int ka = s0 * SEG, kb = min(k, s1 * SEG);
     int steps = (kb - ka + BK - 1) / BK;
     auto fetch_w = [&](int s) {
-        fetch<TW, Tile::FEATS, THREADS>(Ws + (s % ST) * ROW<TW> * Tile::FEATS, W, m0, m, k, ka + s * BK, kb, vec);
+        fetch<TW, Tile::FEATS, THREADS>(Ws + (s % ST) * ROW<TW> * Tile::FEATS, W, m0, m, k, ka + s * BK, kb, w_bytes);
     };
     auto fetch_a = [&](int s) {
-        fetch<TA, Tile::ROWS, THREADS>(As + (s % ST) * ROW<TA> * Tile::ROWS, A, n0, n, k, ka + s * BK, kb, vec);
+        fetch<TA, Tile::ROWS, THREADS>(As + (s % ST) * ROW<TA> * Tile::ROWS, A, n0, n, k, ka + s * BK, kb, a_bytes);
     };
     // early: the first stages' weights are on their way while the kernel before this one ends
     if (!early)
         pdl_wait();
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < ST - 1; s++)
         if (s < steps)
             fetch_w(s);
     if (early)
         pdl_wait();
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < ST - 1; s++) {
         if (s < steps)
             fetch_a(s);
@@ -261,12 +295,12 @@ gemm_simt_join_kernel(const float *part, float *__restrict__ out, long long coun
 // unrolled whole, were the fastest of the tiles tried: 8 x 8 a thread spills, more blocks of fewer registers
 // lose more to waiting than they hide.
 // One B200, float, microseconds (before: blocks of 64 x 64 with 16 values of k a stage, or of 128 features and
-// 16 rows), with the second kernel where k is shared out:
-//   rows 8:   6144 x 2560  18.0 (76.7)   2560 x 4096  13.5 (92.3)   19456 x 2560  49 (112)   151936 x 2560  271 (703)
-//   rows 16:  6144 x 2560  23.0          2560 x 4096  19.2          19456 x 2560  68         151936 x 2560  406
-//   rows 64:  6144 x 2560  70 (166)      2560 x 4096  47 (202)      19456 x 2560  211 (375)  2560 x 9728  121 (475)
-//   rows 300: 6144 x 2560  277 (384)     2560 x 4096  178 (313)     19456 x 2560  742 (1089) 2560 x 9728  426 (738)
-// and 2,048 rows run at 45 TFLOP/s (31).  The error against 64 bits is 2.9e-7 of the result (4.1e-7): a chain is
+// 16 rows), weights from memory, with the second kernel where k is shared out:
+//   rows 8:   6144 x 2560  20.3 (80.3)   2560 x 4096  14.7 (77.3)   19456 x 2560  50.2 (113)   151936 x 2560  272 (702)
+//   rows 16:  6144 x 2560  28.1 (89.4)   2560 x 4096  19.9 (75.2)   19456 x 2560  70.0 (115)   151936 x 2560  361 (725)
+//   rows 64:  6144 x 2560  68.5 (181)    2560 x 4096  45.5 (200)    19456 x 2560  207 (369)    2560 x 9728  117 (472)
+//   rows 300: 6144 x 2560  271 (383)     2560 x 4096  172 (309)     19456 x 2560  724 (1,057)  2560 x 9728  414 (729)
+// and 2,048 rows run at 47 TFLOP/s (31).  The error against 64 bits is 2.9e-7 of the result (4.1e-7): a chain is
 // half as long.
 typedef SimtTile<4, 2, 32, 2, 3> Rows8;
 typedef SimtTile<4, 4, 16, 4, 3> Rows16;
@@ -276,13 +310,25 @@ static_assert(Rows8::FEATS == Rows64::FEATS && Rows16::FEATS == Rows64::FEATS, "
 
 static int simt_segments(int k) { return (k + SEG - 1) / SEG; }
 
+// Rows of the tile that n rows go with.  A single segment cannot be shared out over blocks: 17 to 32 rows are then two
+// tiles of 16, whose blocks are half as long (24 rows, float: 96 x 100 4.6 us against 6.3, 1000 x 100 4.9 against 6.4).
+// With more segments one tile is ahead where there are many (2560 x 9728 49 against 69, 6144 x 2560 33 against 46).
+static int simt_rows(int n, int k)
+{
+    if (n <= 8)
+        return 8;
+    if (n <= 16 || (n <= 32 && simt_segments(k) == 1))
+        return 16;
+    return n <= 32 ? 32 : 64;
+}
+
 // Groups of segments: as few as give every SM a few blocks (four small ones, or two of the others).  The sums
 // that pass through scratch cost 8 bytes a segment, row and feature, the weights 4 bytes x 512 a segment and
 // feature.
 static int simt_groups(int n, int m, int k)
 {
-    int rows = n <= 8 ? Rows8::ROWS : n <= 16 ? Rows16::ROWS : n <= 32 ? Rows32::ROWS : Rows64::ROWS;
-    int feats = n <= 32 && n > 16 ? Rows32::FEATS : Rows64::FEATS;
+    int rows = simt_rows(n, k);
+    int feats = rows == Rows32::ROWS ? Rows32::FEATS : Rows64::FEATS;
     long long tiles = ((long long)m + feats - 1) / feats * (((long long)n + rows - 1) / rows);
     long long want = (rows < 64 ? 4 : 2) * (long long)sm_count();
     int segments = simt_segments(k);
@@ -291,12 +337,26 @@ static int simt_groups(int n, int m, int k)
     return (int)((want + tiles - 1) / tiles < segments ? (want + tiles - 1) / tiles : segments);
 }
 
+// The widest copy (16, 8 or 4 bytes; 2: none) that every row of k values from p on starts and ends at a multiple of,
+// for each operand by itself.  One B200, 2,560 features, rows 8 | 300 | 1,000, microseconds (before: value by value
+// unless both operands could go by 16 bytes):
+//   float            k = 2561   16.9 (104)    131 (379)   390 (1,318)
+//   bfloat16, float  k = 2564   15.6 (101)    130 (498)   392 (1,052)
+//   bfloat16         k = 2561   34.5 (83.9)   206 (374)   570 (954)
+template <typename T> static int copy_bytes(const void *p, int k)
+{
+    unsigned long long at = (unsigned long long)(uintptr_t)p | (unsigned long long)k * sizeof(T);
+    return at % 16 == 0 ? 16 : at % 8 == 0 ? 8 : at % 4 == 0 ? 4 : 2;
+}
+
 template <typename TA, typename TW, typename Tile>
-static bool simt_launch(const void *A, const void *W, float *out, int n, int m, int k, int groups, bool vec,
+static bool simt_launch(const void *A, const void *W, float *out, int n, int m, int k, int groups,
                         bool early, cudaStream_t st)
 {
     static unsigned long long done = 0, done_parts = 0;
-    constexpr int smem = Tile::template smem<TA, TW>();
+    // (no more blocks an SM than simt_groups counts on: bfloat16 weights would let seven in, and the SMs then end
+    // apart: 8 rows, float by bfloat16, 6144 x 2560, 18.2 us against 14.3)
+    constexpr int smem = Tile::template smem<TA, TW>() > (56 << 10) ? Tile::template smem<TA, TW>() : 56 << 10;
     long long row_tiles = ((long long)n + Tile::ROWS - 1) / Tile::ROWS;
     long long tiles = row_tiles * (((long long)m + Tile::FEATS - 1) / Tile::FEATS);
     if (tiles > 0x7fffffffll)
@@ -306,12 +366,12 @@ static bool simt_launch(const void *A, const void *W, float *out, int n, int m, 
         if (!allow_dynamic_smem(gemm_simt_kernel<TA, TW, Tile, true>, smem, done_parts))
             return false;
         launch(gemm_simt_kernel<TA, TW, Tile, true>, grid, Tile::THREADS, smem, st, (const TA *)A, (const TW *)W, out,
-               n, m, k, (int)row_tiles, vec, early);
+               n, m, k, (int)row_tiles, copy_bytes<TA>(A, k), copy_bytes<TW>(W, k), early);
     } else {
         if (!allow_dynamic_smem(gemm_simt_kernel<TA, TW, Tile, false>, smem, done))
             return false;
         launch(gemm_simt_kernel<TA, TW, Tile, false>, grid, Tile::THREADS, smem, st, (const TA *)A, (const TW *)W, out,
-               n, m, k, (int)row_tiles, vec, early);
+               n, m, k, (int)row_tiles, copy_bytes<TA>(A, k), copy_bytes<TW>(W, k), early);
     }
     return true;
 }
@@ -320,15 +380,14 @@ template <typename TA, typename TW>
 static bool simt_pick(const void *A, const void *W, float *out, int n, int m, int k, int groups, bool early,
                       cudaStream_t st)
 {
-    bool vec = ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0) && k % (16 / (int)sizeof(TA)) == 0 &&
-               k % (16 / (int)sizeof(TW)) == 0;
-    if (n <= 8)
-        return simt_launch<TA, TW, Rows8>(A, W, out, n, m, k, groups, vec, early, st);
-    if (n <= 16)
-        return simt_launch<TA, TW, Rows16>(A, W, out, n, m, k, groups, vec, early, st);
-    if (n <= 32)
-        return simt_launch<TA, TW, Rows32>(A, W, out, n, m, k, groups, vec, early, st);
-    return simt_launch<TA, TW, Rows64>(A, W, out, n, m, k, groups, vec, early, st);
+    int rows = simt_rows(n, k);
+    if (rows == Rows8::ROWS)
+        return simt_launch<TA, TW, Rows8>(A, W, out, n, m, k, groups, early, st);
+    if (rows == Rows16::ROWS)
+        return simt_launch<TA, TW, Rows16>(A, W, out, n, m, k, groups, early, st);
+    if (rows == Rows32::ROWS)
+        return simt_launch<TA, TW, Rows32>(A, W, out, n, m, k, groups, early, st);
+    return simt_launch<TA, TW, Rows64>(A, W, out, n, m, k, groups, early, st);
 }
 
 }  // namespace jb

@@ -127,6 +127,30 @@ def test_gemm_simt_rows(adt, wdt, m, k):
         assert torch.equal(ops().linear(a_dev[:n].contiguous(), w_dev, force_simt=True)[0], whole[:n]), n
 
 
+@pytest.mark.parametrize("adt", DTYPES)
+@pytest.mark.parametrize("wdt", DTYPES)
+@pytest.mark.parametrize("k", [96, 100, 511, 514, 1030])
+def test_gemm_simt_copies(adt, wdt, k):
+    """Rows that start and end at multiples of 16, 8, 4 or 2 bytes, by their length and by where the operand starts:
+    the copies differ, the bits do not."""
+    m = 70
+    a, w = rnd(40, k, dtype=adt).to(DEV), rnd(m, k, dtype=wdt, seed=3).to(DEV)
+
+    def moved(t, by):
+        flat = torch.full((t.numel() + 8,), math.nan, dtype=t.dtype, device=DEV)
+        out = flat[by:by + t.numel()].view(t.shape)
+        out.copy_(t)
+        return out
+
+    bound = (258 + k // 512) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    whole = ops().linear(a, w, force_simt=True)[0]
+    assert ((whole.double() - a.double() @ w.double().T).abs() <= bound).all()
+    for ao, wo in ((1, 0), (0, 1), (2, 4), (4, 2), (3, 3)):
+        for n in (1, 9, 20, 40):
+            got = ops().linear(moved(a[:n], ao), moved(w, wo), force_simt=True)[0]
+            assert torch.equal(got, whole[:n]), (ao, wo, n)
+
+
 @pytest.mark.parametrize("odt", DTYPES)
 def test_swiglu(odt):
     n, ff = 7, 300
