@@ -288,12 +288,11 @@ gemm_simt_join_kernel(const float *part, float *__restrict__ out, long long coun
 
 // Which tile: rows up to 8, 16 and 32 stand in one tile, so that a weight is read once; more rows in tiles of 64.
 //
-// Up to 16 rows the weights' bytes are the bound.  A narrow tile (64 features) keeps many blocks on an SM, each
-// with two stages of 16 KB on their way; every multiply-add takes its weight from shared memory, and the reads of
+// Up to 16 rows the weights' bytes are the bound.  A narrow tile (64 features) leaves room for three blocks on an SM,
+// each with two stages of 16 KB on their way; every multiply-add takes its weight from shared memory, and the reads of
 // weights (twice per block of 8 rows) are what is fullest.  From 32 rows on the multiply-adds are the bound
 // (72.7 TFLOP/s is what this instruction gives); four to eight rows and four features a thread, the stage
-// unrolled whole, were the fastest of the tiles tried: 8 x 8 a thread spills, more blocks of fewer registers
-// lose more to waiting than they hide.
+// unrolled whole, were the fastest of the tiles tried (8 x 8 a thread, more blocks of fewer registers).
 // One B200, float, microseconds (before: blocks of 64 x 64 with 16 values of k a stage, or of 128 features and
 // 16 rows), weights from memory, with the second kernel where k is shared out:
 //   rows 8:   6144 x 2560  20.3 (80.3)   2560 x 4096  14.7 (77.3)   19456 x 2560  50.2 (113)   151936 x 2560  272 (702)
@@ -322,15 +321,17 @@ static int simt_rows(int n, int k)
     return n <= 32 ? 32 : 64;
 }
 
-// Groups of segments: as few as give every SM a few blocks (four small ones, or two of the others).  The sums
-// that pass through scratch cost 8 bytes a segment, row and feature, the weights 4 bytes x 512 a segment and
-// feature.
+// Groups of segments: as few as give every SM the blocks that fit it at a time (by shared memory three of 8 or 16 rows,
+// two of 64), and for tiles of 32 rows, of which two fit, twice as many.  8 | 16 rows, 2560 x 9728, float: 28.7 | 40.7
+// us; counting four of them a SM, whose last round is nearly empty, 32.4 | 44.2.  24 rows, 2560 x 9728 and 19456 x 2560:
+// 49 and 107; counting two of them a SM 74 and 121.  The sums that pass through scratch cost 8 bytes a segment, row and
+// feature, the weights 4 bytes x 512 a segment and feature.
 static int simt_groups(int n, int m, int k)
 {
     int rows = simt_rows(n, k);
     int feats = rows == Rows32::ROWS ? Rows32::FEATS : Rows64::FEATS;
     long long tiles = ((long long)m + feats - 1) / feats * (((long long)n + rows - 1) / rows);
-    long long want = (rows < 64 ? 4 : 2) * (long long)sm_count();
+    long long want = (rows < 32 ? 3 : rows == 32 ? 4 : 2) * (long long)sm_count();
     int segments = simt_segments(k);
     if (tiles >= want)
         return 1;
@@ -354,8 +355,8 @@ static bool simt_launch(const void *A, const void *W, float *out, int n, int m, 
                         bool early, cudaStream_t st)
 {
     static unsigned long long done = 0, done_parts = 0;
-    // (no more blocks an SM than simt_groups counts on: bfloat16 weights would let seven in, and the SMs then end
-    // apart: 8 rows, float by bfloat16, 6144 x 2560, 18.2 us against 14.3)
+    // (no more than four blocks an SM: bfloat16 weights would let seven in, and the SMs then end apart: 8 rows, float
+    // by bfloat16, 6144 x 2560, 18.2 us against 14.3)
     constexpr int smem = Tile::template smem<TA, TW>() > (56 << 10) ? Tile::template smem<TA, TW>() : 56 << 10;
     long long row_tiles = ((long long)n + Tile::ROWS - 1) / Tile::ROWS;
     long long tiles = row_tiles * (((long long)m + Tile::FEATS - 1) / Tile::FEATS);
