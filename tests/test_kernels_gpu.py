@@ -127,6 +127,19 @@ def test_gemm_simt_rows(adt, wdt, m, k):
         assert torch.equal(ops().linear(a_dev[:n].contiguous(), w_dev, force_simt=True)[0], whole[:n]), n
 
 
+@pytest.mark.parametrize("adt,wdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("m,k", [(76001, 1100), (20000, 2560)])
+def test_gemm_simt_several_segments_a_block(adt, wdt, m, k):
+    """So many features that a block of any tile walks more than one segment: all of them (running totals), or the
+    group it has (their sums side by side in scratch).  Bits and bound as above."""
+    a, w = rnd(67, k, dtype=adt).to(DEV), rnd(m, k, dtype=wdt, seed=3).to(DEV)
+    whole = ops().linear(a, w, force_simt=True)[0]
+    bound = (258 + k // 512) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert ((whole.double() - a.double() @ w.double().T).abs() <= bound).all()
+    for n in (1, 8, 9, 16, 17, 32, 33, 64, 65):
+        assert torch.equal(ops().linear(a[:n].contiguous(), w, force_simt=True)[0], whole[:n]), n
+
+
 @pytest.mark.parametrize("adt", DTYPES)
 @pytest.mark.parametrize("wdt", DTYPES)
 @pytest.mark.parametrize("k", [96, 100, 511, 514, 1030])
