@@ -27,7 +27,6 @@
 namespace jb {
 
 constexpr int ATT_CHUNK = 128;  // positions per partial (two pages)
-constexpr int ATT_GT = 4;       // query heads a warp carries at once
 
 // The 16 values of a head that lane c of LPK holds lie in groups of 16 bytes (4 floats, 8 bfloat16), LPK groups
 // apart, so that the lanes of a key read its row in whole lines.  Place of value j; the load of all 16 from a row
@@ -79,14 +78,50 @@ __host__ __device__ inline size_t part_at(size_t row, int nh, int h, int max_chu
     return ((row * nh + h) * max_chunks + ci) * (size_t)(hd + 2);
 }
 
+// The sums over a warp's key groups of a lane's 16 values.  Every round halves the values that a lane goes on with, so
+// that a value is added up once and not in every lane: lane bit LPK takes the upper eight, the next bit the upper four
+// of those, and so on; LEFT values of each are left, from first_left(lane) on.
+template <int LPK> constexpr int LEFT = LPK > 1 ? LPK / 2 : 1;
+
+template <int LPK> __device__ __forceinline__ int first_left(int lane)
+{
+    int first = 0;
+#pragma unroll
+    for (int off = LPK, n = 8; off < 32 && n > 0; off <<= 1, n >>= 1)
+        first += lane & off ? n : 0;
+    return first;
+}
+
+template <int LPK> __device__ __forceinline__ void sum_groups(float (&o)[16], int lane)
+{
+#pragma unroll
+    for (int off = LPK, n = 8; off < 32; off <<= 1, n >>= 1) {
+        bool up = lane & off;
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (j < n) {
+                float keep = up ? o[j + n] : o[j], give = up ? o[j] : o[j + n];
+                o[j] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+            }
+        if (n == 0)
+            o[0] += __shfl_xor_sync(0xffffffffu, o[0], off);
+    }
+}
+
 // LPK lanes share one key (16 values of the head each); 32 / LPK keys a step.  What bounds it is the chain of a
-// warp's steps and, with every place taken, the instructions of each: a warp has a quarter of a chunk, loads run
-// a pair of steps ahead and take whole lines, and the weights are made once all scores are there, a lane a key,
-// instead of a rescaling of the sums at every key.  One B200, float, 32 heads on 8 of 128, microseconds (before:
-// a warp per chunk, key by key, each step's loads waited for): 8 rows at context 2,048 52 -> 41; two layers of a
-// prompt of 300 rows with their products 5,750 -> 3,708, of which the products' share is 1,800; 36 layers of a
-// prompt of 2,048 rows 636 -> 460 ms.
-template <typename T, int LPK>
+// warp's steps and, with every place taken, the instructions of each: the unit of work is a quarter of a chunk; its
+// scores are made a pair of steps at a time, its values are asked for a pair of steps ahead, both in whole lines, and
+// the weights are made once all scores are there, a lane a key, instead of a rescaling of the sums at every key.
+// A warp has a quarter and a block a (row, chunk), whose quarters are joined through shared memory; or (ALONE) a warp
+// has a (row, chunk) and goes through its quarters in order.  The sums are the same, bit for bit.  GT: query heads of
+// the group that a warp carries at once.
+// One B200, float, microseconds with the merge (a warp per chunk, key by key | the quarters joined a head after the
+// other, all of a group of four carried always | now):
+//   32 heads on 8 of 128:  8 rows at context 2,048   64 | 42 | 36      64 rows at 1,000          245 | 134 | 116
+//                          a prompt of 300 rows     211 | 110 | 89     one of 1,500              3,125 | 1,878 | 1,539
+//                          one row at position 0    6.0 | 8.8 | 5.8    four prompts of 33 rows   23.0 | 31.5 | 18.7
+//   16 heads of 64, 4 of 16: a prompt of 1,500 rows  2,970 | 2,311 | 1,162  and  278 | 403 | 146
+template <typename T, int LPK, int GT, bool ALONE>
 __global__ void __launch_bounds__(128)
 attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
                     const T *__restrict__ v_cache, const int32_t *__restrict__ row_pos,
@@ -97,20 +132,23 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
                     const float *__restrict__ slopes, int keep_first,
                     const float *__restrict__ score_bias)
 {
-    constexpr int KPW = 32 / LPK;
-    constexpr int QUARTER = ATT_CHUNK / 4;
+    constexpr int KPW = 32 / LPK, U = LPK > 1 ? 2 : 1;
+    constexpr int QUARTER = ATT_CHUNK / 4, QS = ALONE ? 4 : 1;
     static_assert(QUARTER == 32 && PAGE % QUARTER == 0, "a lane for every key of a quarter, all of one page");
-    __shared__ float so[4][ATT_GT][LPK * 16], sml[4][ATT_GT][2], sc[4][ATT_GT][QUARTER];
+    // weights, and largest score and sum of weights, by warp and (ALONE) quarter; a block's quarters' weighted values
+    __shared__ float sc[4][QS][GT][QUARTER], sml[4][QS][GT][3], so[ALONE ? 1 : 4][GT][ALONE ? 1 : LPK * 16];
     pdl_trigger();
     pdl_wait();
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    size_t item = blockIdx.x;
+    size_t item = ALONE ? (size_t)blockIdx.x * 4 + warp : blockIdx.x;
+    if (ALONE && item >= (size_t)n_rows * max_chunks)
+        return;
     int lrow = (int)(item / max_chunks), ci = (int)(item % max_chunks);
     int row = row0 + lrow;
     int kvh = blockIdx.y;
     int group = nh / nkv;
-    int g0 = blockIdx.z * ATT_GT;
-    int gt = min(ATT_GT, group - g0);
+    int g0 = blockIdx.z * GT;
+    int gt = min(GT, group - g0);
     int h0 = kvh * group + g0;
 
     int pos = row_pos[row];
@@ -131,37 +169,38 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
         t0 = max(lo, c * ATT_CHUNK);
         t1 = min(pos, c * ATT_CHUNK + ATT_CHUNK - 1);
     }
-
-    // this warp's quarter of the chunk
-    t0 = max(t0, c * ATT_CHUNK + warp * QUARTER);
-    t1 = min(t1, c * ATT_CHUNK + warp * QUARTER + QUARTER - 1);
+    // the quarters that the row sees something of, and those of them that this warp has
+    const int qa = t0 <= t1 ? (t0 - c * ATT_CHUNK) / QUARTER : 0, qb = t0 <= t1 ? (t1 - c * ATT_CHUNK) / QUARTER : -1;
+    const int wa = ALONE ? qa : warp, wb = ALONE ? qb : warp >= qa && warp <= qb ? warp : warp - 1;
 
     int cidx = lane % LPK, ks = lane / LPK;
     constexpr int GS = 16 / sizeof(T);
     const bool vec_k = hd % GS == 0 && (((uintptr_t)q | (uintptr_t)k_cache) & 15) == 0;
     const bool vec_v = vd % GS == 0 && v_ld % GS == 0 && ((uintptr_t)v_cache & 15) == 0;
     const int32_t *bt = block_table + (size_t)row_seq[row] * bt_stride;
+    const float inv_cap = softcap > 0.0f ? 1.0f / softcap : 0.0f;
 
-    // The warp's 32 keys in three passes: their scores (LPK lanes a key, a pair of steps' keys on their way
+    // A quarter's keys in three passes: their scores (LPK lanes a key, a pair of steps' keys on their way
     // together) into shared memory; a lane a key for the largest, the weights and their sum; the values.
     // Every key has its place by its position, so the sums' order is the row's own.
-    const int base = c * ATT_CHUNK + warp * QUARTER;
-    constexpr int U = LPK > 1 ? 2 : 1;
-    const size_t at0 = t0 <= t1 ? ((size_t)bt[base / PAGE] * nkv + kvh) * PAGE + base % PAGE : 0;   // (a quarter lies in one page)
-    auto seen = [&](int key) { return base + key >= t0 && base + key <= t1; };
-    auto ask = [&](const T *rows, int ld, int count, bool vec, int key, float (&x)[16]) {
-        if (seen(key)) {
-            load16<T, LPK>(rows + (at0 + key) * ld, x, cidx, count, vec);
+    // (a quarter lies in one page, a chunk in two)
+    const int page0 = qa < 2 && qb >= 0 ? bt[c * (ATT_CHUNK / PAGE)] : 0, page1 = qb >= 2 ? bt[c * (ATT_CHUNK / PAGE) + 1] : 0;
+    static_assert(ATT_CHUNK == 2 * PAGE, "two pages a chunk");
+    auto first_row = [&](int qi) { return ((size_t)(qi < 2 ? page0 : page1) * nkv + kvh) * PAGE + (qi & 1) * QUARTER; };
+    auto ask = [&](const T *rows, int ld, int count, bool vec, int key, int ka, int kb, float (&x)[16]) {
+        if (key >= ka && key <= kb) {
+            load16<T, LPK>(rows + (size_t)key * ld, x, cidx, count, vec);
         } else {
 #pragma unroll
             for (int j = 0; j < 16; j++)
                 x[j] = 0.0f;
         }
     };
-    if (t0 <= t1) {
-        float qv[ATT_GT][16];
+    float vv[U][16];
+    if (wa <= wb) {
+        float qv[GT][16];
 #pragma unroll
-        for (int g = 0; g < ATT_GT; g++) {
+        for (int g = 0; g < GT; g++) {
 #pragma unroll
             for (int j = 0; j < 16; j++)
                 qv[g][j] = 0.0f;
@@ -169,127 +208,221 @@ attn_partial_kernel(const T *__restrict__ q, const T *__restrict__ k_cache,
                 load16<T, LPK>(q + ((size_t)row * nh + h0 + g) * hd, qv[g], cidx, hd, vec_k);
         }
 #pragma unroll 1
-        for (int st = 0; st < LPK; st += U) {
-            float kv[U][16];
-#pragma unroll
-            for (int u = 0; u < U; u++)
-                ask(k_cache, hd, hd, vec_k, (st + u) * KPW + ks, kv[u]);
-#pragma unroll
-            for (int u = 0; u < U; u++)
-#pragma unroll
-                for (int g = 0; g < ATT_GT; g++) {
-                    float d = 0.0f;
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        d = fmaf(qv[g][j], kv[u][j], d);
-#pragma unroll
-                    for (int off = 1; off < LPK; off <<= 1)
-                        d += __shfl_xor_sync(0xffffffffu, d, off);
-                    if (cidx == 0)
-                        sc[warp][g][(st + u) * KPW + ks] = d;
-                }
-        }
-    }
-    float vv[U][16];
-#pragma unroll
-    for (int u = 0; u < U; u++)
-        ask(v_cache, v_ld, vd, vec_v, u * KPW + ks, vv[u]);
-    __syncwarp();
-    float o[ATT_GT][16], m[ATT_GT], l[ATT_GT];
-    const float inv_cap = softcap > 0.0f ? 1.0f / softcap : 0.0f;
-#pragma unroll
-    for (int g = 0; g < ATT_GT; g++) {
-        bool on = g < gt && seen(lane);
-        float x = -INFINITY;
-        if (on) {
-            x = sc[warp][g][lane] * scale;
-            if (head_scale != nullptr)          // a head's own factor on its scores
-                x *= head_scale[h0 + g];
-            if (softcap > 0.0f)
-                x = softcap * tanhf(x * inv_cap);
-            if (slopes != nullptr)              // slope * distance is taken off the score of a key that far back
-                x -= slopes[h0 + g] * (float)(pos - (base + lane));
-        }
-        float p;
-        if (score_bias != nullptr) {
-            // the sigmoid of the score and a number per head is the key's weight: no maximum, no sum of weights
-            m[g] = -INFINITY;
-            l[g] = 0.0f;
-            p = on ? 1.0f / (1.0f + expf(-(x + score_bias[h0 + g]))) : 0.0f;
-        } else {
-            m[g] = warp_max(x);         // (passes over NaN: a NaN score makes its own weight, and so the sums, NaN)
-            p = on && x != -INFINITY ? expf(x - m[g]) : 0.0f;
-            l[g] = warp_sum(p);
-        }
-        sc[warp][g][lane] = p;
-#pragma unroll
-        for (int j = 0; j < 16; j++)
-            o[g][j] = 0.0f;
-    }
-    __syncwarp();
-    if (t0 <= t1) {
+        for (int qi = wa; qi <= wb; qi++) {
+            const int base = c * ATT_CHUNK + qi * QUARTER, at = ALONE ? qi : 0;
+            const int ka = max(t0 - base, 0), kb = min(t1 - base, QUARTER - 1);     // the keys of it that are seen
+            const size_t row_at = first_row(qi);
 #pragma unroll 1
-        for (int st = 0; st < LPK; st += U) {
+            for (int st = ka / KPW / U * U; st <= kb / KPW; st += U) {
+                float kv[U][16];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    ask(k_cache + row_at * hd, hd, hd, vec_k, (st + u) * KPW + ks, ka, kb, kv[u]);
+#pragma unroll
+                for (int u = 0; u < U; u++)
+#pragma unroll
+                    for (int g = 0; g < GT; g++) {
+                        float d = 0.0f;
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            d = fmaf(qv[g][j], kv[u][j], d);
+#pragma unroll
+                        for (int off = 1; off < LPK; off <<= 1)
+                            d += __shfl_xor_sync(0xffffffffu, d, off);
+                        if (cidx == 0)
+                            sc[warp][at][g][(st + u) * KPW + ks] = d;
+                    }
+            }
+            if (!ALONE) {
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    ask(v_cache + row_at * v_ld, v_ld, vd, vec_v, (ka / KPW / U * U + u) * KPW + ks, ka, kb, vv[u]);
+            }
+            __syncwarp();
+            const bool on = lane >= ka && lane <= kb;
+            float x[GT], m[GT], l[GT];
+#pragma unroll
+            for (int g = 0; g < GT; g++)
+                x[g] = on && g < gt ? sc[warp][at][g][lane] * scale : -INFINITY;
+            if (head_scale != nullptr) {        // a head's own factor on its scores
+#pragma unroll
+                for (int g = 0; g < GT; g++)
+                    if (on && g < gt)
+                        x[g] *= head_scale[h0 + g];
+            }
+            if (softcap > 0.0f) {
+#pragma unroll
+                for (int g = 0; g < GT; g++)
+                    if (on && g < gt)
+                        x[g] = softcap * tanhf(x[g] * inv_cap);
+            }
+            if (slopes != nullptr) {            // slope * distance is taken off the score of a key that far back
+#pragma unroll
+                for (int g = 0; g < GT; g++)
+                    if (on && g < gt)
+                        x[g] -= slopes[h0 + g] * (float)(pos - (base + lane));
+            }
+            if (score_bias != nullptr) {
+                // the sigmoid of the score and a number per head is the key's weight: no maximum, no sum of weights
+#pragma unroll
+                for (int g = 0; g < GT; g++) {
+                    m[g] = -INFINITY;
+                    l[g] = 0.0f;
+                    x[g] = on && g < gt ? 1.0f / (1.0f + expf(-(x[g] + score_bias[h0 + g]))) : 0.0f;
+                }
+            } else {
+                // (the largest passes over NaN: a NaN score makes its own weight, and so the sums, NaN)
+#pragma unroll
+                for (int g = 0; g < GT; g++)
+                    m[g] = warp_max(x[g]);
+#pragma unroll
+                for (int g = 0; g < GT; g++) {
+                    x[g] = x[g] != -INFINITY ? expf(x[g] - m[g]) : 0.0f;
+                    l[g] = warp_sum(x[g]);
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < GT; g++) {
+                sc[warp][at][g][lane] = x[g];
+                if (lane == 0) {
+                    sml[warp][at][g][0] = m[g];
+                    sml[warp][at][g][1] = l[g];
+                }
+            }
+        }
+    }
+    __syncwarp();
+    // a quarter's factor in the whole: e^(its largest score - the largest of all)
+    auto factor = [&](float m_w, float m) { return score_bias != nullptr ? 1.0f : m == -INFINITY ? 0.0f : expf(m_w - m); };
+    // the partial's place
+    auto place = [&](int g) { return part + part_at((size_t)lrow, nh, h0 + g, max_chunks, ci, vd); };
+    if (ALONE) {
+        // a lane a quarter and head
+        int qi = lane / GT, g = lane % GT;
+        bool live = qi >= qa && qi <= qb;
+        float m_w = live ? sml[warp][qi & 3][g][0] : -INFINITY, m = m_w, sum = 0.0f;
+#pragma unroll
+        for (int off = GT; off < 4 * GT; off <<= 1)
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+        float f = factor(m_w, m), lf = live ? sml[warp][qi & 3][g][1] : 0.0f;
+        if (live)
+            sml[warp][qi & 3][g][2] = f;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            float f_w = __shfl_sync(0xffffffffu, f, w * GT + g), l_w = __shfl_sync(0xffffffffu, lf, w * GT + g);
+            sum = w >= qa && w <= qb ? fmaf(l_w, f_w, sum) : sum;
+        }
+        if (lane < gt) {
+            place(g)[0] = m;
+            place(g)[1] = sum;
+        }
+        __syncwarp();
+    }
+    const int j0 = first_left<LPK>(lane);
+    float all[GT][LEFT<LPK>];
+    if (ALONE) {
+#pragma unroll
+        for (int g = 0; g < GT; g++)
+#pragma unroll
+            for (int j = 0; j < LEFT<LPK>; j++)
+                all[g][j] = 0.0f;
+    }
+#pragma unroll 1
+    for (int qi = wa; qi <= wb; qi++) {
+        const int base = c * ATT_CHUNK + qi * QUARTER, at = ALONE ? qi : 0;
+        const int ka = max(t0 - base, 0), kb = min(t1 - base, QUARTER - 1), sa = ka / KPW / U * U;
+        const T *rows = v_cache + first_row(qi) * v_ld;
+        float o[GT][16];
+#pragma unroll
+        for (int g = 0; g < GT; g++)
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+                o[g][j] = 0.0f;
+        if (ALONE) {
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                ask(rows, v_ld, vd, vec_v, (sa + u) * KPW + ks, ka, kb, vv[u]);
+        }
+#pragma unroll 1
+        for (int st = sa; st <= kb / KPW; st += U) {
             float now[U][16];
 #pragma unroll
             for (int u = 0; u < U; u++)
 #pragma unroll
                 for (int j = 0; j < 16; j++)
                     now[u][j] = vv[u][j];
-            if (st + U < LPK) {
+            if (st + U <= kb / KPW) {
 #pragma unroll
                 for (int u = 0; u < U; u++)
-                    ask(v_cache, v_ld, vd, vec_v, (st + U + u) * KPW + ks, vv[u]);
+                    ask(rows, v_ld, vd, vec_v, (st + U + u) * KPW + ks, ka, kb, vv[u]);
             }
 #pragma unroll
             for (int u = 0; u < U; u++)
 #pragma unroll
-                for (int g = 0; g < ATT_GT; g++) {
-                    float p = sc[warp][g][(st + u) * KPW + ks];
+                for (int g = 0; g < GT; g++) {
+                    float p = sc[warp][at][g][(st + u) * KPW + ks];
 #pragma unroll
                     for (int j = 0; j < 16; j++)
                         o[g][j] = fmaf(p, now[u][j], o[g][j]);
                 }
         }
-    }
-    // the 32 / LPK key groups of the warp into one
 #pragma unroll
-    for (int off = LPK; off < 32; off <<= 1)
+        for (int g = 0; g < GT; g++) {
+            sum_groups<LPK>(o[g], lane);
+            if (ALONE) {
+                float f = sml[warp][at][g][2];
 #pragma unroll
-        for (int g = 0; g < ATT_GT; g++)
+                for (int j = 0; j < LEFT<LPK>; j++)
+                    all[g][j] = fmaf(o[g][j], f, all[g][j]);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 16; j++)
-                o[g][j] += __shfl_xor_sync(0xffffffffu, o[g][j], off);
-
-    // the quarters into one, in order
-    if (ks == 0) {
-#pragma unroll
-        for (int g = 0; g < ATT_GT; g++) {
-            if (lane == 0) {
-                sml[warp][g][0] = m[g];
-                sml[warp][g][1] = l[g];
+                for (int j = 0; j < LEFT<LPK>; j++)
+                    so[ALONE ? 0 : warp][g][ALONE ? 0 : lane_value<T, LPK>(cidx, j0 + j)] = o[g][j];
             }
-#pragma unroll
-            for (int j = 0; j < 16; j++)
-                so[warp][g][lane_value<T, LPK>(cidx, j)] = o[g][j];
         }
     }
-    __syncthreads();
-    for (int g = 0; g < gt; g++) {
-        float mn = fmaxf(fmaxf(sml[0][g][0], sml[1][g][0]), fmaxf(sml[2][g][0], sml[3][g][0]));
-        float f[4], sum = 0.0f;
+
+    if (ALONE) {
+#pragma unroll
+        for (int g = 0; g < GT; g++)
+#pragma unroll
+            for (int j = 0; j < LEFT<LPK>; j++) {
+                int d = lane_value<T, LPK>(cidx, j0 + j);
+                if (g < gt && d < vd && (LPK > 1 || lane < 16))
+                    place(g)[2 + d] = all[g][j];
+            }
+    } else {
+        // the quarters into one, in order: 4 / GT warps a head
+        __syncthreads();
+        constexpr int WARPS = 4 / GT;
+        const int g = warp / WARPS;
+        float m_w[4], f[4], m = -INFINITY, sum = 0.0f;
 #pragma unroll
         for (int w = 0; w < 4; w++) {
-            f[w] = score_bias != nullptr ? 1.0f : mn == -INFINITY ? 0.0f : expf(sml[w][g][0] - mn);
-            sum = fmaf(sml[w][g][1], f[w], sum);
+            m_w[w] = w >= qa && w <= qb ? sml[w][0][g][0] : -INFINITY;
+            m = fmaxf(m, m_w[w]);
         }
-        float *dst = part + part_at((size_t)lrow, nh, h0 + g, max_chunks, ci, vd);
-        if (threadIdx.x == 0) {
-            dst[0] = mn;
-            dst[1] = sum;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            f[w] = factor(m_w[w], m);
+            sum = w >= qa && w <= qb ? fmaf(sml[w][0][g][1], f[w], sum) : sum;
         }
-        for (int d = threadIdx.x; d < vd; d += 128)
-            dst[2 + d] = fmaf(so[3][g][d], f[3], fmaf(so[2][g][d], f[2], fmaf(so[1][g][d], f[1], so[0][g][d] * f[0])));
+        if (g < gt) {
+            float *dst = place(g);
+            int first = warp % WARPS * 32 + lane;
+            if (first == 0) {
+                dst[0] = m;
+                dst[1] = sum;
+            }
+#pragma unroll 4
+            for (int d = first; d < vd; d += WARPS * 32) {
+                float o = 0.0f;
+#pragma unroll
+                for (int w = 0; w < 4; w++)
+                    o = w >= qa && w <= qb ? fmaf(so[ALONE ? 0 : w][g][ALONE ? 0 : d], f[w], o) : o;
+                dst[2 + d] = o;
+            }
+        }
     }
 }
 
@@ -775,6 +908,16 @@ __global__ void attn_merge_kernel(const float *__restrict__ part,
         out[((size_t)row * nh + h) * hd + d] = from_f<T>(o / l);
 }
 
+// Whether a warp takes a (row, chunk) by itself.  Rows that all end in their first chunk leave most of a block's warps
+// without a quarter, and where there are so many that blocks come in several waves (about three fit an SM) the idle
+// warps' places count: prompts of 4 x 33 rows, 32 heads on 8, float, microseconds alone | a block a row: heads of 128
+// 18.7 | 23.6, heads of 80 16.9 | 22.1; bfloat16, heads of 80 19.4 | 27.5.  Fewer rows: 8 at context 40 12.0 | 8.4, 64 at 100
+// 25.8 | 19.8.  Heads of up to 32 values do not gain (6.2 | 5.4), nor do those of more than 128 (16.3 | 14.0).
+static bool attn_rows_alone(long long blocks, int lpk, int max_chunks)
+{
+    return max_chunks == 1 && (lpk == 4 || lpk == 8) && blocks >= 7ll * sm_count();
+}
+
 template <typename T>
 static int attention_typed(const T *q, const T *k_cache, const T *v_cache, const int32_t *row_pos,
                            const int32_t *row_seq, const int32_t *block_table, int bt_stride,
@@ -791,20 +934,29 @@ static int attention_typed(const T *q, const T *k_cache, const T *v_cache, const
     size_t items = (size_t)n_rows * max_chunks;
     if (items > 0x7fffffff)
         return JB_EINVAL;
-    dim3 grid((unsigned)items, nkv, (group + ATT_GT - 1) / ATT_GT);
-#define JB_ATT(L)                                                                            \
-    launch(attn_partial_kernel<T, L>, grid, 128, 0, st, q, k_cache, v_cache, row_pos, row_seq, \
-           block_table, bt_stride, part, row0, n_rows, nh, nkv, hd, vd, window, scale,        \
+    const int gt = group < 3 ? group : 4, parts = (group + gt - 1) / gt;
+    const bool alone = attn_rows_alone((long long)items * nkv * parts, lpk, max_chunks);
+    dim3 grid((unsigned)(alone ? (items + 3) / 4 : items), nkv, parts);
+#define JB_ATT_AS(L, G, A)                                                                       \
+    launch(attn_partial_kernel<T, L, G, A>, grid, 128, 0, st, q, k_cache, v_cache, row_pos, row_seq, \
+           block_table, bt_stride, part, row0, n_rows, nh, nkv, hd, vd, window, scale,           \
            head_scale, max_chunks, v_ld, softcap, slopes, keep_first, score_bias)
-    switch (lpk) {
-    case 1: JB_ATT(1); break;
-    case 2: JB_ATT(2); break;
-    case 4: JB_ATT(4); break;
-    case 8: JB_ATT(8); break;
-    case 16: JB_ATT(16); break;
-    case 32: JB_ATT(32); break;
+#define JB_ATT(L, A)                                                                             \
+    if (gt == 1) JB_ATT_AS(L, 1, A);                                                             \
+    else if (gt == 2) JB_ATT_AS(L, 2, A);                                                        \
+    else JB_ATT_AS(L, 4, A)
+    switch (alone ? -lpk : lpk) {
+    case 1: JB_ATT(1, false); break;
+    case 2: JB_ATT(2, false); break;
+    case 4: JB_ATT(4, false); break;
+    case 8: JB_ATT(8, false); break;
+    case 16: JB_ATT(16, false); break;
+    case 32: JB_ATT(32, false); break;
+    case -4: JB_ATT(4, true); break;
+    case -8: JB_ATT(8, true); break;
     default: return JB_EINVAL;
     }
+#undef JB_ATT_AS
 #undef JB_ATT
     if (cudaGetLastError() != cudaSuccess)
         return JB_ELAUNCH;

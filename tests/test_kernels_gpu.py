@@ -299,6 +299,51 @@ def test_attention_keeps_what_is_not_finite(dtype, what, nh, nkv, hd, window):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nh,nkv,hd,vd", [(16, 16, 64, 64), (16, 8, 128, 100), (32, 8, 80, 80), (21, 7, 40, 128), (40, 8, 96, 20)])
+@pytest.mark.parametrize("window", [0, 20])
+def test_attention_many_short_rows(dtype, nh, nkv, hd, vd, window):
+    """Rows that all end in their first chunk, so many that a warp takes a row by itself: the bits of each row are
+    those of a step that has it beside few others, under everything that a mixer does to its scores."""
+    n = 340                                             # rows x KV heads: beyond seven blocks an SM
+    pos = torch.from_numpy(np.random.default_rng(4).integers(0, 128, n).astype(np.int32))
+    pos[:8] = torch.tensor([0, 31, 32, 63, 64, 95, 96, 127], dtype=torch.int32)
+    seq = torch.arange(n, dtype=torch.int32) % 3
+    q = rnd(n, nh, hd, dtype=dtype).to(DEV)
+    kc, vc = rnd(6, nkv, 64, hd, dtype=dtype, seed=1).to(DEV), rnd(6, nkv, 64, vd, dtype=dtype, seed=2).to(DEV)
+    bt = torch.tensor([[5, 0], [2, 4], [1, 3]], dtype=torch.int32).to(DEV)
+    head = rnd(nh, seed=3).to(DEV)
+    for extra in ({}, dict(head_scale=head.abs() + 0.5, sink=head), dict(softcap=2.0, slopes=head.abs()),
+                  dict(score_bias=head)):
+        def run(rows):
+            return ops().attention(q[rows].contiguous(), kc, vc, pos[rows].to(DEV), seq[rows].to(DEV), bt, window,
+                                   1 / math.sqrt(hd), 1, force_simt=True, value_dim=vd, **extra)
+        whole = run(slice(0, n))
+        for a in (0, 4, 100, n - 4):
+            assert torch.equal(run(slice(a, a + 4)), whole[a:a + 4]), (extra.keys(), a)
+        # against the definition, in 64 bits
+        rows = torch.arange(0, n, 17)
+        sel = bt.cpu()[seq[rows].long()].long().to(DEV)
+        k = kc[sel].double().permute(0, 2, 1, 3, 4).reshape(len(rows), nkv, 128, hd).repeat_interleave(nh // nkv, 1)
+        v = vc[sel].double().permute(0, 2, 1, 3, 4).reshape(len(rows), nkv, 128, vd).repeat_interleave(nh // nkv, 1)
+        s = torch.einsum("nhd,nhkd->nhk", q[rows].double(), k) / math.sqrt(hd)
+        p_, key = pos[rows].to(DEV)[:, None, None], torch.arange(128, device=DEV)
+        s = s * extra["head_scale"][:, None] if "head_scale" in extra else s
+        s = 2.0 * torch.tanh(s / 2.0) if "softcap" in extra else s
+        s = s - extra["slopes"][:, None] * (p_ - key) if "slopes" in extra else s
+        seen = (key <= p_) & (key > p_ - window if window else key >= 0)
+        if "score_bias" in extra:
+            w = torch.sigmoid(s + head[:, None]) * seen
+        else:
+            e = torch.where(seen, s, -math.inf)
+            top = e.amax(-1, keepdim=True)
+            e = (e - top).exp()
+            w = e / (e.sum(-1, keepdim=True) + ((head[:, None] - top).exp() if "sink" in extra else 0))
+        want = torch.einsum("nhk,nhkd->nhd", w, v)
+        tol = 5e-6 if dtype == torch.float32 else 2 ** -8
+        assert ((whole[rows].double() - want).abs().max() <= tol * want.abs().max()), extra.keys()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n0,n1,hd,nh,nkv", [(25, 15, 48, 6, 2), (300, 58, 128, 6, 2), (3, 1, 16, 6, 2),
                                              (40, 9, 32, 5, 1), (17, 30, 64, 9, 3),
                                              (9, 11, 256, 3, 3), (6, 3, 80, 4, 2),
