@@ -843,7 +843,8 @@ __device__ __forceinline__ void merge_partials(const float *__restrict__ base, s
     o *= a;
 #pragma unroll
     for (int u = 0; u < N; u++) {
-        float w = c0 + u < n_chunks ? expf(mc[u] - mn) : 0.0f;
+        // (an empty partial has weight 0 also where all up to here are empty)
+        float w = c0 + u < n_chunks && mc[u] != -INFINITY ? expf(mc[u] - mn) : 0.0f;
         l = fmaf(lc[u], w, l);
         o = fmaf(oc[u], w, o);
     }

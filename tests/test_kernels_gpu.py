@@ -344,6 +344,24 @@ def test_attention_many_short_rows(dtype, nh, nkv, hd, vd, window):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("keep_first", [2048, 4096, 4200, 9000])
+def test_attention_many_kept_tokens_before_the_window_moves(dtype, keep_first):
+    """Rows that still see everything have the kept first tokens in their window: the partials of the kept chunks,
+    more than the merge takes at a time, are all empty and change nothing."""
+    n, nh, nkv, hd, window = 200, 4, 2, 80, 10000
+    q, k, v = rnd(n, nh, hd, dtype=dtype), rnd(n, nkv, hd, dtype=dtype, seed=1), rnd(n, nkv, hd, dtype=dtype, seed=2)
+    kc, vc, bt = paged(k, v, 9)
+    pos, seq = torch.arange(n, dtype=torch.int32).to(DEV), torch.zeros(n, dtype=torch.int32).to(DEV)
+
+    def run(window, keep_first):
+        mc = ops().attention_kept_chunks(window, keep_first) + (n - 1) // ops().attention_chunk() + 1
+        return ops().attention(q.to(DEV), kc.to(DEV), vc.to(DEV), pos, seq, bt.to(DEV), window, 1 / math.sqrt(hd), mc,
+                               force_simt=True, keep_first=keep_first)
+
+    assert torch.equal(run(window, keep_first), run(0, 0))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n0,n1,hd,nh,nkv", [(25, 15, 48, 6, 2), (300, 58, 128, 6, 2), (3, 1, 16, 6, 2),
                                              (40, 9, 32, 5, 1), (17, 30, 64, 9, 3),
                                              (9, 11, 256, 3, 3), (6, 3, 80, 4, 2),
