@@ -14,12 +14,18 @@ VALUES = [7, 0, -3, 2 ** 31 - 1]
 @pytest.mark.parametrize("kind", [int, float, str, np.int64, np.int32, np.float64, Fraction, torch.tensor])
 @pytest.mark.parametrize("hold", [list, tuple, iter, lambda v: (x for x in v), lambda v: dict.fromkeys(v).keys()])
 def test_packing(kind, hold):
-    assert list(_ints(hold([kind(v) for v in VALUES]))) == VALUES
+    for values in (VALUES, VALUES + [11, 12, 13]):          # short lists are packed another way
+        assert list(_ints(hold([kind(v) for v in values]))) == values
 
 
 @pytest.mark.parametrize("values", [np.array(VALUES), np.array(VALUES, dtype=np.float64), torch.tensor(VALUES), range(5)])
 def test_packing_of_arrays(values):
     assert list(_ints(values)) == [int(v) for v in values]
+
+
+@pytest.mark.parametrize("n", [1, 4, 5, 40])
+def test_packing_beyond_32_bits(n):
+    assert list(_ints([2 ** 40 + 5] * n)) == [5] * n        # the low 32 bits, as a C int takes them
 
 
 def test_packing_of_nothing_leaves_a_place():
