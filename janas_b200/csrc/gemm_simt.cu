@@ -1,7 +1,8 @@
 // out[n, m] = A[n, k] . W[m, k]^T with plain float multiply-adds.
 //
-// This is the matrix product of the true 32-bit path and the fallback for
-// shapes and type mixes the tensor-core kernel refuses.  Every output value is
+// This is the matrix product of the true 32-bit path for weights that are small
+// or whose rows TMA does not take (the others: gemm_f32_tc.cu), and the fallback
+// for shapes and type mixes the bfloat16 tensor-core kernel refuses.  Every output value is
 // computed by one fixed recipe, whatever n is and wherever the row lies in the
 // batch, so a row's result is the same bits however the tokens are cut into
 // steps: k is cut into segments of SEG values at fixed places; within a segment

@@ -424,15 +424,14 @@ EncodeTiled tensor_map_encoder()
     return fn;
 }
 
-// A [rows, k] bfloat16 row-major matrix, read in boxes of box_rows x 64 with the
-// 128-byte swizzle; what lies outside the matrix reads as zero.
-static bool tensor_map(const void *ptr, int rows, int k, int box_rows, CUtensorMap *out)
+bool tensor_map_2d(const void *ptr, int rows, int k, int box_rows, int box_k, CUtensorMapDataType type,
+                   CUtensorMap *out)
 {
-    typedef std::tuple<const void *, int, int, int> Key;
+    typedef std::tuple<const void *, int, int, int, int> Key;
     static std::map<Key, CUtensorMap> cache;
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
-    Key key(ptr, rows, k, box_rows);
+    Key key(ptr, rows, k, box_rows, (int)type);
     auto it = cache.find(key);
     if (it != cache.end()) {
         *out = it->second;
@@ -442,11 +441,11 @@ static bool tensor_map(const void *ptr, int rows, int k, int box_rows, CUtensorM
     if (!enc)
         return false;
     cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    cuuint64_t strides[1] = {(cuuint64_t)k * (type == CU_TENSOR_MAP_DATA_TYPE_FLOAT32 ? 4 : 2)};
+    cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUtensorMap map;
-    if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box,
+    if (enc(&map, type, 2, const_cast<void *>(ptr), dims, strides, box,
             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
@@ -455,6 +454,11 @@ static bool tensor_map(const void *ptr, int rows, int k, int box_rows, CUtensorM
     cache[key] = map;
     *out = map;
     return true;
+}
+
+static bool tensor_map(const void *ptr, int rows, int k, int box_rows, CUtensorMap *out)
+{
+    return tensor_map_2d(ptr, rows, k, box_rows, BK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out);
 }
 
 template <int BN, int MT, int EPI>
@@ -688,8 +692,9 @@ extern "C" int jb_gemm_tc_gated(const void *A, const void *W, void *out_act, int
 #undef JB_SWIGLU_HALF
 }
 
-// Reads and clears the error word: 0, or which wait ran out first (1: a free
-// stage, 2: a loaded stage, 3: the accumulator, 4: a load in flight).
+// Reads and clears the error words of the products: 0, or which wait ran out first (1: a free
+// stage, 2: a loaded stage, 3: the accumulator, 4: a load in flight; from 20 on: in the product of
+// floats, gemm_f32_tc.cu).
 // Synchronizes the device.
 // A wait that nothing ends, to show that a bounded wait runs out as it should: one
 // warp, one mbarrier that no thread and no copy ever arrives at, the products' own
@@ -731,5 +736,6 @@ extern "C" int jb_gemm_tc_error(void)
         return JB_ELAUNCH;
     if (v != 0)
         cudaMemcpyToSymbol(g_gemm_tc_error, &zero, sizeof zero);
-    return v;
+    int f = jb_gemm_f32_tc_error();
+    return v != 0 ? v : f > 0 ? f + 20 : f;
 }

@@ -305,6 +305,12 @@ int jb_attn_tc_error(void);
 long long jb_gemm_simt_scratch(int n, int m, int k);
 int jb_gemm_simt(const void *A, int a_dt, const void *W, int w_dt, float *out, int n, int m, int k,
                  float *scratch, int early, cudaStream_t st);
+int jb_gemm_f32_tc_ok(const void *W, int m, int k);
+long long jb_gemm_f32_tc_scratch(int n, int m, int k);
+int jb_gemm_f32_tc_launches(int n, int m, int k);
+int jb_gemm_f32_tc(const void *A, const void *W, float *out, int n, int m, int k, float *scratch,
+                   int early, cudaStream_t st);
+int jb_gemm_f32_tc_error(void);
 int jb_gemm_tc_ok(const void *A, const void *W, int n, int m, int k);
 int jb_gemm_tc_splits(int n, int m, int k);
 int jb_gemm_tc(const void *A, const void *W, float *out, int n, int m, int k, int splits,

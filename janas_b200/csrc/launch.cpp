@@ -602,6 +602,20 @@ int linear_parts(long long n, long long m, long long k) {
     return jb_gemm_tc_splits((int)n, (int)m, (int)k);
 }
 
+// out = a . w^T whole: floats by the tensor cores in parts where that kernel takes the weight's shape (whatever the
+// rows are, so that a row's bits do not depend on the batch), anything else by plain multiply-adds
+static void plain_product(Device &d, const void *a, DType a_dt, const void *w, DType w_dt, float *out, int n, int m,
+                          int k, bool force_simt, const char *what) {
+    bool parts = !force_simt && a_dt == F32 && w_dt == F32 && jb_gemm_f32_tc_ok(w, m, k) != 0;
+    long long need = parts ? jb_gemm_f32_tc_scratch(n, m, k) : jb_gemm_simt_scratch(n, m, k);
+    Buf scratch;
+    if (need > 0) scratch = d.pool.get((size_t)need * 4);
+    if (parts)
+        check(jb_gemm_f32_tc(a, w, out, n, m, k, scratch.as<float>(), 1, d.stream), what, jb_gemm_f32_tc_launches(n, m, k));
+    else
+        check(jb_gemm_simt(a, a_dt, w, w_dt, out, n, m, k, scratch.as<float>(), 1, d.stream), what, need > 0 ? 2 : 1);
+}
+
 Stack linear(Device &d, const void *a, DType a_dt, long long n, long long k, const DevTensor &w,
              bool whole, bool force_simt, int splits) {
     need_float(a_dt, "activations");
@@ -621,11 +635,7 @@ Stack linear(Device &d, const void *a, DType a_dt, long long n, long long k, con
     }
     out.S = 1;
     out.buf = d.pool.get((size_t)n * (size_t)m * 4);
-    long long need = jb_gemm_simt_scratch(ni, mi, ki);
-    Buf scratch;
-    if (need > 0) scratch = d.pool.get((size_t)need * 4);
-    check(jb_gemm_simt(a, a_dt, w.ptr, w.dt, out.data(), ni, mi, ki, scratch.as<float>(), 1, d.stream),
-          "linear", need > 0 ? 2 : 1);
+    plain_product(d, a, a_dt, w.ptr, w.dt, out.data(), ni, mi, ki, force_simt, "linear");
     return out;
 }
 
@@ -647,9 +657,6 @@ HeadStack linear_heads(Device &d, const void *a, DType a_dt, int H, long long n,
     out.S = tc ? jb_gemm_tc_splits(ni, mi, ki) : 1;
     size_t one = (size_t)out.S * (size_t)n * (size_t)out.m;
     out.buf = d.pool.get(std::max<size_t>((size_t)H * one * 4, 16));
-    long long need = tc ? 0 : jb_gemm_simt_scratch(ni, mi, ki);
-    Buf scratch;
-    if (need > 0) scratch = d.pool.get((size_t)need * 4);
     if (tc) {
         check(jb_gemm_tc_heads(a, w.ptr, out.data(), ni, mi, ki, out.S, H, d.stream), "linear_heads (tcgen05)");
         return out;
@@ -657,8 +664,7 @@ HeadStack linear_heads(Device &d, const void *a, DType a_dt, int H, long long n,
     for (int h = 0; h < H && n > 0; h++) {
         const char *ah = (const char *)a + h * a_head, *wh = (const char *)w.ptr + h * w_head;
         float *oh = out.data() + (size_t)h * one;
-        check(jb_gemm_simt(ah, a_dt, wh, w.dt, oh, ni, mi, ki, scratch.as<float>(), 1, d.stream),
-              "linear_heads", need > 0 ? 2 : 1);
+        plain_product(d, ah, a_dt, wh, w.dt, oh, ni, mi, ki, false, "linear_heads");
     }
     return out;
 }

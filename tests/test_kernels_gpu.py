@@ -164,6 +164,47 @@ def test_gemm_simt_copies(adt, wdt, k):
             assert torch.equal(got, whole[:n]), (ao, wo, n)
 
 
+@pytest.mark.parametrize("m,k", [(512, 1024), (513, 1028), (640, 2560), (2560, 9728), (19000, 1100)])
+def test_gemm_f32_parts(m, k):
+    """The product of floats in parts: every tile of tokens at its edges, features and k that fill no tile or block,
+    tiles taken whole and shared out by segments.  A row's bits do not depend on the rows beside it.  The error: what
+    is left out is 2^-26 of a product; an MMA cuts off at most 17 terms at 2^-24 of the block's sum, four of them do at
+    its full size and the others at 2^-8 of it or less; then one rounding a block and segment."""
+    a, w = rnd(321, k).to(DEV), rnd(m, k, seed=3).to(DEV)
+    L = ops().lib()
+    assert L.jb_gemm_f32_tc_ok(w.data_ptr(), m, k)
+    whole = ops().linear(a, w)[0]
+    blocks = -(-k // 64)
+    bound = (1 + 17 * 5 + 2 * blocks) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert ((whole.double() - a.double() @ w.double().T).abs() <= bound).all()
+    for n in (1, 15, 16, 17, 32, 33, 64, 65, 96, 97, 128, 129, 160, 161, 256, 320):
+        assert torch.equal(ops().linear(a[:n].contiguous(), w)[0], whole[:n]), n
+    flat = torch.empty(40 * k + 1, device=DEV)
+    moved = flat[1:].view(40, k)                   # rows that start at no multiple of 16 bytes
+    moved.copy_(a[:40])
+    for n in (9, 40):
+        assert torch.equal(ops().linear(moved[:n], w)[0], whole[:n]), n
+    assert ops().gemm_tc_error() == 0
+
+
+@pytest.mark.parametrize("n", [5, 70])
+def test_gemm_f32_parts_not_finite(n):
+    """Infinities, NaN and floats too large for a part, in single rows and features: the products of the plain kernel
+    there, and nothing of them anywhere else."""
+    a, w = rnd(n, 1100).to(DEV), rnd(600, 1100, seed=3).to(DEV)
+    clean = ops().linear(a, w)[0]
+    b, v = a.clone(), w.clone()
+    b[1, 700], b[2, 2], b[3, 1099], v[11, 600], v[12, 5] = math.inf, math.nan, 3.4e38, -math.inf, 3.4e38
+    got, want = ops().linear(b, v)[0], ops().linear(b, v, force_simt=True)[0]
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[want.isinf()], want[want.isinf()])
+    rows = [r for r in range(n) if r not in (1, 2, 3)]
+    cols = [c for c in range(600) if c not in (11, 12)]
+    assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+    ok = want.isfinite()
+    assert ((got - want)[ok].abs() <= 2e-6 * (b.double().abs() @ v.double().abs().T)[ok]).all()
+
+
 @pytest.mark.parametrize("odt", DTYPES)
 def test_swiglu(odt):
     n, ff = 7, 300
