@@ -121,7 +121,7 @@ attn_tc_rows_kernel(const __grid_constant__ CUtensorMap map_q,
     uint32_t *tmem_slot = (uint32_t *)(bars + 9);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
 
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     int kvh = blockIdx.y;
 
     // ---- what this CTA works on: a run of chunks of one decoded token
@@ -161,7 +161,7 @@ attn_tc_rows_kernel(const __grid_constant__ CUtensorMap map_q,
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    uint32_t tmem = *tmem_slot;
+    uint32_t tmem = warp_uniform(*tmem_slot);
     uint32_t tmem_s = tmem, tmem_pv = tmem + AT_KEYS;
     int *err = &g_attn_tc_error;
     // q, the keys and the values were written by the kernel before this one
@@ -209,45 +209,41 @@ attn_tc_rows_kernel(const __grid_constant__ CUtensorMap map_q,
                 if (armed & (1u << s))
                     mbar_wait(bar(1 + s), (last_parity >> s) & 1, &never, err, 4);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // --------------------------------------------------------------- MMAs
+        // (the whole warp waits and one lane is elected to issue: see tc_mma4)
+        auto all = [](bool there) { return __all_sync(0xffffffffu, there) != 0; };
         constexpr uint32_t idesc_s = instr_desc_bf16(AT_ROWS, AT_KEYS, false);
         constexpr uint32_t idesc_pv = instr_desc_bf16(AT_ROWS, HD, true);
-        bool ok = mbar_wait(bar(0), 0, abort, err, 2);
-        uint32_t q_a = smem_u32(q_s), p_a = smem_u32(p_s);
+        bool ok = all(mbar_wait(bar(0), 0, abort, err, 2));
+        const uint64_t dq = smem_desc_sw128(smem_u32(q_s), 16, 1024), dp = smem_desc_sw128(smem_u32(p_s), 16, 1024);
         for (int it = 0; it < n_chunks && ok; it++) {
             int s = it % AT_STAGES;
             uint32_t ph = (it / AT_STAGES) & 1;
-            ok = mbar_wait(bar(1 + s), ph, abort, err, 3);
+            ok = all(mbar_wait(bar(1 + s), ph, abort, err, 3));
             if (!ok)
                 break;
             tc_fence_after();
             uint32_t k_a = smem_u32(kv_s + s * Cfg::KV_STAGE);
-            uint32_t v_a = k_a + NB * BLK_BYTES;
-            // S = Q K^T over the head's values, 16 at a time
+            const uint64_t dk = smem_desc_sw128(k_a, 16, 1024), dv = smem_desc_sw128(k_a + NB * BLK_BYTES, BLK_BYTES, 1024);
+            // S = Q K^T over the head's values, 64 at a time
 #pragma unroll
-            for (int kk = 0; kk < HD / 16; kk++) {
-                uint32_t off = (kk / 4) * BLK_BYTES + (kk % 4) * 32;
-                tc_mma(tmem_s, smem_desc_sw128(q_a + off, 16, 1024),
-                       smem_desc_sw128(k_a + off, 16, 1024), idesc_s, kk != 0);
-            }
-            tc_commit(bar(5));
-            ok = mbar_wait(bar(6), it & 1, abort, err, 5);       // P is in shared memory
+            for (int bb = 0; bb < HD / 64; bb++)
+                tc_mma4<2, 2>(tmem_s, dq + bb * (BLK_BYTES >> 4), dk + bb * (BLK_BYTES >> 4), idesc_s, bb != 0);
+            tc_commit_warp(bar(5));
+            ok = all(mbar_wait(bar(6), it & 1, abort, err, 5));       // P is in shared memory
             if (ok && it > 0)
-                ok = mbar_wait(bar(8), (it - 1) & 1, abort, err, 6);   // the last PV was read
+                ok = all(mbar_wait(bar(8), (it - 1) & 1, abort, err, 6));   // the last PV was read
             if (!ok)
                 break;
             tc_fence_after();
-            // PV = P V over the chunk's keys, 16 at a time; V is MN-major: blocks of 64
+            // PV = P V over the chunk's keys, 64 at a time; V is MN-major: blocks of 64
             // values BLK_BYTES apart, groups of eight keys 1024 bytes apart
 #pragma unroll
-            for (int kk = 0; kk < AT_KEYS / 16; kk++) {
-                uint32_t p_off = (kk / 4) * BLK_BYTES + (kk % 4) * 32;
-                tc_mma(tmem_pv, smem_desc_sw128(p_a + p_off, 16, 1024),
-                       smem_desc_sw128(v_a + kk * 16 * 128, BLK_BYTES, 1024), idesc_pv, kk != 0);
-            }
-            tc_commit(bar(7));
-            tc_commit(bar(3 + s));
+            for (int bb = 0; bb < AT_KEYS / 64; bb++)
+                tc_mma4<2, 128>(tmem_pv, dp + bb * (BLK_BYTES >> 4), dv + bb * 512, idesc_pv, bb != 0);
+            tc_commit_warp(bar(7));
+            tc_commit_warp(bar(3 + s));
         }
     } else if (warp >= 2) {
         // ------------------------------------------------------------ row threads
@@ -436,7 +432,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
     uint32_t *tmem_slot = (uint32_t *)(bars + 15);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
 
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         prefetch_tensor_map(&map_q);
         prefetch_tensor_map(&map_k);
@@ -483,7 +479,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    uint32_t tmem = *tmem_slot;
+    uint32_t tmem = warp_uniform(*tmem_slot);
     int *err = &g_attn_tc_error;
     // q, the keys and the values were written by the kernel before this one
     pdl_trigger();
@@ -533,8 +529,10 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
                 if (armed & (1u << s))
                     mbar_wait(bar(1 + s), (last_parity >> s) & 1, &never, err, 24);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // --------------------------------------------------------------- MMAs
+        // (the whole warp waits and one lane is elected to issue: see tc_mma4)
+        auto all = [](bool there) { return __all_sync(0xffffffffu, there) != 0; };
         constexpr uint32_t idesc_s = instr_desc_bf16(AT_ROWS, AT_KEYS, false);
         constexpr uint32_t idesc_pv = instr_desc_bf16(AT_ROWS, VD, true);
         int tiles = has_b ? 2 : 1;
@@ -543,31 +541,29 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
         // asked for a whole chunk before it is needed.
         auto unit_k = [&](int j) { return j == 0 ? 0 : 2 * j - 1; };
         auto unit_v = [&](int j) { return j == n_chunks - 1 ? 2 * n_chunks - 1 : 2 * j + 2; };
-        bool ok = mbar_wait(bar(0), 0, abort, err, 22);
+        bool ok = all(mbar_wait(bar(0), 0, abort, err, 22));
         // the scores of chunk `it` of block t; the chunk's keys are in unit 2 it
         auto issue_s = [&](int it, int t) {
             // one descriptor per operand; the steps along k are added to its address
-            // field (16-byte units), so that the one issuing thread has little to compute
+            // field (16-byte units)
             uint64_t dq = smem_desc_sw128(smem_u32(q_s + t * Cfg::Q_TILE), 16, 1024);
             uint64_t dk = smem_desc_sw128(
                 smem_u32(kv_s + (unit_k(it) % PF_UNITS) * Cfg::UNIT), 16, 1024);
 #pragma unroll
-            for (int kk = 0; kk < KD / 16; kk++) {
-                uint64_t off = (uint64_t)(((kk / 4) * BLK_BYTES + (kk % 4) * 32) >> 4);
-                tc_mma(tmem + t * AT_KEYS, dq + off, dk + off, idesc_s, kk != 0);
-            }
-            tc_commit(bar(7 + t));
+            for (int bb = 0; bb < KD / 64; bb++)
+                tc_mma4<2, 2>(tmem + t * AT_KEYS, dq + bb * (BLK_BYTES >> 4), dk + bb * (BLK_BYTES >> 4), idesc_s, bb != 0);
+            tc_commit_warp(bar(7 + t));
         };
         auto keys_there = [&](int it) {
             int u = unit_k(it);
-            bool there = mbar_wait(bar(1 + u % PF_UNITS), (u / PF_UNITS) & 1, abort, err, 23);
+            bool there = all(mbar_wait(bar(1 + u % PF_UNITS), (u / PF_UNITS) & 1, abort, err, 23));
             tc_fence_after();
             return there;
         };
         if (ok && (ok = keys_there(0))) {
             for (int t = 0; t < tiles; t++)
                 issue_s(0, t);
-            tc_commit(bar(4 + 0));                 // the keys' unit is free once these are done
+            tc_commit_warp(bar(4 + 0));                 // the keys' unit is free once these are done
         }
         for (int it = 0; it < n_chunks && ok; it++) {
             // the next chunk's scores as soon as the row threads hold this chunk's in
@@ -575,7 +571,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
             if (it + 1 < n_chunks) {
                 ok = keys_there(it + 1);
                 for (int t = 0; t < tiles && ok; t++) {
-                    ok = mbar_wait(bar(13 + t), it & 1, abort, err, 30);
+                    ok = all(mbar_wait(bar(13 + t), it & 1, abort, err, 30));
                     if (!ok)
                         break;
                     tc_fence_after();
@@ -583,27 +579,25 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
                 }
                 if (!ok)
                     break;
-                tc_commit(bar(4 + unit_k(it + 1) % PF_UNITS));
+                tc_commit_warp(bar(4 + unit_k(it + 1) % PF_UNITS));
             }
             int uv = unit_v(it), sv = uv % PF_UNITS;
             for (int t = 0; t < tiles && ok; t++) {
-                ok = mbar_wait(bar(9 + t), it & 1, abort, err, 25);               // P is there
+                ok = all(mbar_wait(bar(9 + t), it & 1, abort, err, 25));               // P is there
                 if (ok && t == 0)
-                    ok = mbar_wait(bar(1 + sv), (uv / PF_UNITS) & 1, abort, err, 26);   // the values
+                    ok = all(mbar_wait(bar(1 + sv), (uv / PF_UNITS) & 1, abort, err, 26));   // the values
                 if (!ok)
                     break;
                 tc_fence_after();
                 uint64_t dv = smem_desc_sw128(smem_u32(kv_s + sv * Cfg::UNIT), BLK_BYTES, 1024);
                 uint64_t dp = smem_desc_sw128(smem_u32(p_s + t * Cfg::P_TILE), 16, 1024);
 #pragma unroll
-                for (int kk = 0; kk < AT_KEYS / 16; kk++) {
-                    uint64_t p_off = (uint64_t)(((kk / 4) * BLK_BYTES + (kk % 4) * 32) >> 4);
-                    tc_mma(tmem + 2 * AT_KEYS + t * VD, dp + p_off, dv + (uint64_t)(kk * 128),
-                           idesc_pv, (it | kk) != 0);
-                }
-                tc_commit(bar(11 + t));
+                for (int bb = 0; bb < AT_KEYS / 64; bb++)
+                    tc_mma4<2, 128>(tmem + 2 * AT_KEYS + t * VD, dp + bb * (BLK_BYTES >> 4), dv + bb * 512, idesc_pv,
+                                    (it | bb) != 0);
+                tc_commit_warp(bar(11 + t));
                 if (t == tiles - 1)
-                    tc_commit(bar(4 + sv));        // the values' unit is free
+                    tc_commit_warp(bar(4 + sv));        // the values' unit is free
             }
         }
     } else if (warp >= 2) {
@@ -915,7 +909,7 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
     float *red_m = (float *)(tmem_slot + 4);   // [4 warps][16 heads]
     float *red_l = red_m + 4 * DQ_N;
 
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         prefetch_tensor_map(&map_k);
         prefetch_tensor_map(&map_v);
@@ -972,7 +966,7 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    uint32_t tmem = *tmem_slot;
+    uint32_t tmem = warp_uniform(*tmem_slot);
     uint32_t tmem_s = tmem, tmem_pv = tmem + 2 * DQ_N;    // S: two buffers of 16 columns
     int *err = &g_attn_tc_error;
     // q and the keys and values of position q_pos were written by the kernel before
@@ -1147,54 +1141,51 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
                 if (armed & (1u << s))
                     mbar_wait(bar(1 + s), (last_parity >> s) & 1, &never, err, 14);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // --------------------------------------------------------------- MMAs
+        // (the whole warp waits and one lane is elected to issue: see tc_mma4)
+        auto all = [](bool there) { return __all_sync(0xffffffffu, there) != 0; };
         constexpr uint32_t idesc_s = instr_desc_bf16(AT_KEYS, DQ_N, false, false);
         constexpr uint32_t idesc_pv = instr_desc_bf16(HD, DQ_N, false, true);
-        uint32_t q_a = smem_u32(q_s), p_a = smem_u32(p_s);
+        const uint64_t dq = smem_desc_sw128(smem_u32(q_s), 16, 1024);
         // S^T of chunk `it` into S buffer it % 2
         auto issue_s = [&](int it) -> bool {
             int u = 2 * it, s = u % DQ_UNITS;
-            if (!mbar_wait(bar(1 + s), (u / DQ_UNITS) & 1, abort, err, 13))
+            if (!all(mbar_wait(bar(1 + s), (u / DQ_UNITS) & 1, abort, err, 13)))
                 return false;
             tc_fence_after();
-            uint32_t k_a = smem_u32(kv_s + s * DQ_UNIT);
+            uint64_t dk = smem_desc_sw128(smem_u32(kv_s + s * DQ_UNIT), 16, 1024);
 #pragma unroll
-            for (int kk = 0; kk < HD / 16; kk++)
-                tc_mma(tmem_s + (it & 1) * DQ_N,
-                       smem_desc_sw128(k_a + (kk / 4) * BLK_BYTES + (kk % 4) * 32, 16, 1024),
-                       smem_desc_sw128(q_a + (kk / 4) * DQ_BLK + (kk % 4) * 32, 16, 1024),
-                       idesc_s, kk != 0);
-            tc_commit(bar(7 + (it & 1)));
-            tc_commit(bar(4 + s));              // the keys' unit is free once these are done
+            for (int bb = 0; bb < HD / 64; bb++)
+                tc_mma4<2, 2>(tmem_s + (it & 1) * DQ_N, dk + bb * (BLK_BYTES >> 4), dq + bb * (DQ_BLK >> 4), idesc_s, bb != 0);
+            tc_commit_warp(bar(7 + (it & 1)));
+            tc_commit_warp(bar(4 + s));              // the keys' unit is free once these are done
             return true;
         };
-        bool ok = mbar_wait(bar(0), 0, abort, err, 12) && issue_s(0);
+        bool ok = all(mbar_wait(bar(0), 0, abort, err, 12)) && issue_s(0);
         for (int it = 0; it < n_chunks && ok; it++) {
             // the next chunk's scores are computed while the row threads work on this
             // one's; its S buffer was read out before P of chunk it - 1 was ready
             if (it + 1 < n_chunks)
                 ok = issue_s(it + 1);
-            ok = ok && mbar_wait(bar(9 + (it & 1)), (it >> 1) & 1, abort, err, 15);   // P is there
+            ok = ok && all(mbar_wait(bar(9 + (it & 1)), (it >> 1) & 1, abort, err, 15));   // P is there
             if (ok && it > 0)
-                ok = mbar_wait(bar(12), (it - 1) & 1, abort, err, 16);   // the last O^T was read
+                ok = all(mbar_wait(bar(12), (it - 1) & 1, abort, err, 16));   // the last O^T was read
             if (!ok)
                 break;
             tc_fence_after();
             int u = 2 * it + 1, s = u % DQ_UNITS;
-            ok = mbar_wait(bar(1 + s), (u / DQ_UNITS) & 1, abort, err, 19);   // the values are there
+            ok = all(mbar_wait(bar(1 + s), (u / DQ_UNITS) & 1, abort, err, 19));   // the values are there
             if (!ok)
                 break;
             tc_fence_after();
-            uint32_t v_a = smem_u32(kv_s + s * DQ_UNIT);
-            uint32_t pb = p_a + (it & 1) * 2 * DQ_BLK;
+            uint64_t dv = smem_desc_sw128(smem_u32(kv_s + s * DQ_UNIT), BLK_BYTES, 1024);
+            uint64_t dp = smem_desc_sw128(smem_u32(p_s + (it & 1) * 2 * DQ_BLK), 16, 1024);
 #pragma unroll
-            for (int kk = 0; kk < AT_KEYS / 16; kk++)
-                tc_mma(tmem_pv, smem_desc_sw128(v_a + kk * 16 * 128, BLK_BYTES, 1024),
-                       smem_desc_sw128(pb + (kk / 4) * DQ_BLK + (kk % 4) * 32, 16, 1024),
-                       idesc_pv, kk != 0);
-            tc_commit(bar(11));
-            tc_commit(bar(4 + s));
+            for (int bb = 0; bb < AT_KEYS / 64; bb++)
+                tc_mma4<128, 2>(tmem_pv, dv + bb * 512, dp + bb * (DQ_BLK >> 4), idesc_pv, bb != 0);
+            tc_commit_warp(bar(11));
+            tc_commit_warp(bar(4 + s));
         }
     } else if (warp >= 2) {
         // ---------------------------------------------- key threads / value threads

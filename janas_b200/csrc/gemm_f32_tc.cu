@@ -138,9 +138,7 @@ struct F32Cursor {
 };
 
 // d += a . b over a block's k (64: four MMAs; first: d starts from zero), a in tensor memory (lane: row, a column: two
-// values of k), b in shared memory.  By a whole warp, one lane of which is elected to issue them: in a branch that a
-// single lane takes, and with an instruction and an election for each, the compiler moves every operand into uniform
-// registers each time, and an MMA takes 40 to 55 cycles to issue, up to five times as long as it runs.
+// values of k), b in shared memory.  By a whole warp (see tc_mma4).
 __device__ __forceinline__ void tc_mma_ts_block(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                                 uint32_t accumulate)
 {
@@ -164,17 +162,6 @@ __device__ __forceinline__ void tc_mma_ts_block(uint32_t d_tmem, uint32_t a_tmem
         "}\n"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
-}
-
-__device__ __forceinline__ void tc_commit_elect(uint32_t bar)
-{
-    asm volatile(
-        "{\n\t"
-        ".reg .pred q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
-        "}\n"
-        ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t *r)
@@ -247,7 +234,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * BOXES, a_full = w_empty + 8 * BOXES,
                    done = a_full + 8 * BUFS, b_full = done + 8 * BUFS, b_empty = b_full + 8 * SLOTS,
                    acc_empty = b_empty + 8 * SLOTS;
-    int warp = (int)__reduce_max_sync(0xffffffffu, threadIdx.x >> 5), lane = threadIdx.x & 31;
+    int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         prefetch_tensor_map(&map_w);
         if (!FEW)
@@ -278,8 +265,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // (by a reduction over the warp: a value that the compiler knows to be the same in all lanes)
-    const uint32_t tmem = __reduce_max_sync(0xffffffffu, *tmem_slot), tmem_acc = tmem + BUFS * A_COLS;
+    const uint32_t tmem = warp_uniform(*tmem_slot), tmem_acc = tmem + BUFS * A_COLS;
     pdl_trigger();
 
     // Every role walks the CTA's blocks with a cursor, and the places of a ring with a Ring: the place of the use that is
@@ -351,7 +337,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 } else {
                     // the tokens' parts come as lo, mid, hi, each in a slot of its own, and go as early as they can
                     products(0, slots + slot.at * Cfg::SLOT_BYTES, true);
-                    tc_commit_elect(b_empty + 8 * slot.at);
+                    tc_commit_warp(b_empty + 8 * slot.at);
                     slot.next(SLOTS);
                     const uint32_t mid = slots + slot.at * Cfg::SLOT_BYTES, mid_bar = b_empty + 8 * slot.at;
                     if (!all(full(b_full, slot, 2)))
@@ -365,13 +351,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     tc_fence_after();
                     products(2, hi, false);
                     products(0, mid, false);
-                    tc_commit_elect(mid_bar);
+                    tc_commit_warp(mid_bar);
                     products(1, hi, false);
                     products(0, hi, false);
-                    tc_commit_elect(b_empty + 8 * slot.at);
+                    tc_commit_warp(b_empty + 8 * slot.at);
                     slot.next(SLOTS);
                 }
-                tc_commit_elect(done + 8 * buf.at);
+                tc_commit_warp(done + 8 * buf.at);
                 buf.next(BUFS);
                 accum.next(2);
             }
@@ -379,7 +365,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 // the MMAs in flight, with the limit, before the tensor memory is given back: one more commit,
                 // onto the barrier of the use that is still open
                 volatile int never = 0;
-                tc_commit_elect(done + 8 * buf.at);
+                tc_commit_warp(done + 8 * buf.at);
                 mbar_wait(done + 8 * buf.at, buf.parity, &never, err, 6);
             }
         }

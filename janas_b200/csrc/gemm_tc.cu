@@ -259,7 +259,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 * STAGES + 1);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
 
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         prefetch_tensor_map(&map_w);
         prefetch_tensor_map(&map_a);
@@ -299,7 +299,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    uint32_t tmem = *tmem_slot;
+    uint32_t tmem = warp_uniform(*tmem_slot);
 
     pdl_trigger();
     if (warp == 0 && lane == 0 && nkb > 0) {
@@ -353,29 +353,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (armed & (1u << s))
                     mbar_wait(full0 + 8 * s, (last_parity >> s) & 1, &never, &g_gemm_tc_error, 4);
         }
-    } else if (warp == 1 && lane == 0 && nkb > 0) {
+    } else if (warp == 1 && nkb > 0) {
         // --------------------------------------------------------------- MMAs
+        // (the whole warp waits and one lane is elected to issue: see tc_mma4)
         constexpr uint32_t idesc = instr_desc(BN);
-        bool ok = true;
-        for (int i = 0; i < nkb && ok; i++) {
-            int s = i % STAGES;
-            uint32_t ph = (i / STAGES) & 1;
-            ok = mbar_wait(full0 + 8 * s, ph, abort, &g_gemm_tc_error, 2);
-            if (!ok)
+        int s = 0;
+        uint32_t ph = 0;
+        for (int i = 0; i < nkb; i++) {
+            if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph, abort, &g_gemm_tc_error, 2)))
                 break;
             tc_fence_after();
             uint32_t base = smem_u32(smem + s * Cfg::STAGE_BYTES);
             uint64_t da = smem_desc(base + MT * W_TILE_BYTES);
+            static_assert(BK / 16 == 4, "four MMAs a stage");
 #pragma unroll
-            for (int t = 0; t < MT; t++) {
-                uint64_t dw = smem_desc(base + t * W_TILE_BYTES);
-#pragma unroll
-                for (int kk = 0; kk < BK / 16; kk++)
-                    tc_mma(tmem + t * BN, dw + 2 * kk, da + 2 * kk, idesc, (i | kk) != 0);
+            for (int t = 0; t < MT; t++)
+                tc_mma4<2, 2>(tmem + t * BN, smem_desc(base + t * W_TILE_BYTES), da, idesc, i != 0);
+            tc_commit_warp(empty0 + 8 * s);
+            if (++s == STAGES) {
+                s = 0;
+                ph ^= 1;
             }
-            tc_commit(empty0 + 8 * s);
         }
-        tc_commit(accum);
+        tc_commit_warp(accum);
     } else if (warp >= 2) {
         // ------------------------------------------------------------ epilogue
         int q = warp & 3;                       // the TMEM lanes this warp may read

@@ -91,24 +91,49 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tc_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                       uint32_t idesc, uint32_t accumulate)
+// Four MMAs along k, the operands' descriptors SA and SB (units of 16 bytes) apart; accumulate: whether the first one
+// adds to d.  By a whole warp whose lanes agree on the arguments: one of them is elected to issue.  (In a branch that a
+// single lane takes, or with an election each, every instruction waits for its operands to be moved into uniform
+// registers: 40 to 64 cycles an MMA, measured, where one of 16 tokens runs for about 25 and one of 128 for 64.)
+template <int SA, int SB>
+__device__ __forceinline__ void tc_mma4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                        uint32_t accumulate)
 {
     asm volatile(
         "{\n\t"
-        ".reg .pred p;\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "add.u64 a1, %1, %5;\n\t"
+        "add.u64 a2, a1, %5;\n\t"
+        "add.u64 a3, a2, %5;\n\t"
+        "add.u64 b1, %2, %6;\n\t"
+        "add.u64 b2, b1, %6;\n\t"
+        "add.u64 b3, b2, %6;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n\t"
         "}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(SA), "n"(SB)
         : "memory");
 }
+
+// tc_commit by a whole warp.
+__device__ __forceinline__ void tc_commit_warp(uint32_t bar)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+        "}\n"
+        ::"r"(bar) : "memory");
+}
+
+// A value that all lanes of the warp have, as one that the compiler knows to be the same in all of them.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
 
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, float *v)
 {
