@@ -287,7 +287,8 @@ gemm_simt_join_kernel(const float *part, float *__restrict__ out, long long coun
     }
 }
 
-// Which tile: rows up to 8, 16 and 32 stand in one tile, so that a weight is read once; more rows in tiles of 64.
+// Which tile: rows up to 8, 16 and 32 stand in one tile, so that a weight is read once; more rows in tiles of 64, or of
+// 16 or 8 where those of 64 would be few (simt_rows).
 //
 // Up to 16 rows the weights' bytes are the bound.  A narrow tile (64 features) leaves room for three blocks on an SM,
 // each with two stages of 16 KB on their way; every multiply-add takes its weight from shared memory, and the reads of
@@ -314,13 +315,24 @@ static int simt_segments(int k) { return (k + SEG - 1) / SEG; }
 // tiles of 16, whose blocks are half as long (24 rows, float, us: 96 x 100 3.1 against 5.2, 2560 x 512 11.1 against 17.2, 20000 x 512 26
 // against 31; a head of 151,936 features, which fills the chip either way, 143 against 127).
 // With more segments one tile is ahead where there are many (2560 x 9728 49 against 69, 6144 x 2560 33 against 46).
-static int simt_rows(int n, int k)
+//
+// More rows: tiles of 64 unless those of 16 or 8 are well ahead, which they are where few tiles of 64 leave the chip
+// idle (a block walks its k alone, and one of 8 rows does in 0.4 of the time).  The estimate, in microseconds for a
+// segment of 512: what a block alone takes beside others, and what each block takes of the chip's time; both measured.
+// One B200, us, float, before (tiles of 64) -> now: 96 x 96, 132 rows 5.0 -> 2.1; 448 x 96, 132 rows 5.3 -> 2.4; 96 x 224,
+// 132 rows 8.7 -> 3.6; 512 x 512, 64 rows 16.3 -> 6.4; 2560 x 512, 132 rows 28.7 -> 16.5; 8 x 2560, 300 rows 16.9 -> 11.5.
+static int simt_rows(int n, int m, int k)
 {
     if (n <= 8)
         return 8;
     if (n <= 16 || (n <= 32 && simt_segments(k) == 1))
         return 16;
-    return n <= 32 ? 32 : 64;
+    if (n <= 32)
+        return 32;
+    double columns = ((double)m + Rows64::FEATS - 1) / Rows64::FEATS * simt_segments(k);
+    auto cost = [&](int rows, double alone, double each) { return alone + each * ((n + rows - 1) / rows) * columns; };
+    double c8 = cost(8, 3.8, 0.022), c16 = cost(16, 5.4, 0.031), c64 = cost(64, 9.8, 0.108) * 0.8;
+    return c8 < c16 && c8 < c64 ? 8 : c16 < c64 ? 16 : 64;
 }
 
 // Groups of segments: as few as give every SM the blocks that fit it at a time (by shared memory three of 8 or 16 rows,
@@ -330,7 +342,7 @@ static int simt_rows(int n, int k)
 // feature, the weights 4 bytes x 512 a segment and feature.
 static int simt_groups(int n, int m, int k)
 {
-    int rows = simt_rows(n, k);
+    int rows = simt_rows(n, m, k);
     int feats = rows == Rows32::ROWS ? Rows32::FEATS : Rows64::FEATS;
     long long tiles = ((long long)m + feats - 1) / feats * (((long long)n + rows - 1) / rows);
     long long want = (rows < 32 ? 3 : rows == 32 ? 4 : 2) * (long long)sm_count();
@@ -383,7 +395,7 @@ template <typename TA, typename TW>
 static bool simt_pick(const void *A, const void *W, float *out, int n, int m, int k, int groups, bool early,
                       cudaStream_t st)
 {
-    int rows = simt_rows(n, k);
+    int rows = simt_rows(n, m, k);
     if (rows == Rows8::ROWS)
         return simt_launch<TA, TW, Rows8>(A, W, out, n, m, k, groups, early, st);
     if (rows == Rows16::ROWS)

@@ -164,6 +164,17 @@ def test_gemm_simt_copies(adt, wdt, k):
             assert torch.equal(got, whole[:n]), (ao, wo, n)
 
 
+@pytest.mark.parametrize("m,k", [(96, 96), (70, 516), (320, 100), (640, 512), (5000, 512)])
+def test_gemm_simt_tiles_of_many_rows(m, k):
+    """From 33 rows on the tile goes by rows, features and segments: the bits do not, across the changes."""
+    a, w = rnd(601, k).to(DEV), rnd(m, k, seed=3).to(DEV)
+    whole = ops().linear(a, w, force_simt=True)[0]
+    bound = (258 + k // 512) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert ((whole.double() - a.double() @ w.double().T).abs() <= bound).all()
+    for n in (33, 40, 64, 65, 100, 132, 200, 299, 500):
+        assert torch.equal(ops().linear(a[:n].contiguous(), w, force_simt=True)[0], whole[:n]), n
+
+
 @pytest.mark.parametrize("m,k", [(512, 1024), (513, 1028), (640, 2560), (2560, 9728), (19000, 1100)])
 def test_gemm_f32_parts(m, k):
     """The product of floats in parts: every tile of tokens at its edges, features and k that fill no tile or block,
