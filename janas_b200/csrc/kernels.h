@@ -302,6 +302,7 @@ int jb_attention_merge_gen(const float *scratch, const int32_t *row_pos, void *o
                            int chunks_per_part, const float *sink, int keep_first, int plain_sum,
                            cudaStream_t st);
 int jb_attn_tc_error(void);
+int jb_copy_words(const void *src, void *dst, int n, int src_early, cudaStream_t st);
 long long jb_gemm_simt_scratch(int n, int m, int k);
 int jb_gemm_simt(const void *A, int a_dt, const void *W, int w_dt, float *out, int n, int m, int k,
                  float *scratch, int early, cudaStream_t st);

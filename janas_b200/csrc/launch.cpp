@@ -597,6 +597,10 @@ void rope_table(Device &d, const float *inv, int half, long long n_pos, float *c
     check(jb_rope_table_scaled(cs, sn, inv, as_int(n_pos, "positions"), half, amplitude, d.stream), "rope_table");
 }
 
+void copy_words(Device &d, const void *src, void *dst, long long n, bool src_early) {
+    check(jb_copy_words(src, dst, as_int(n, "words"), src_early ? 1 : 0, d.stream), "copy_words");
+}
+
 // ------------------------------------------------------------------ products
 int linear_parts(long long n, long long m, long long k) {
     return jb_gemm_tc_splits((int)n, (int)m, (int)k);

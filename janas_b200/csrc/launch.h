@@ -47,6 +47,9 @@ namespace ops {
 // how many of the library's kernels have been launched (for measurements)
 long long launches();
 void count_launches(long long n);
+// n 32-bit words between pinned host memory and the device, in the stream's order.  src_early: nothing that may still
+// be running writes src.
+void copy_words(Device &d, const void *src, void *dst, long long n, bool src_early);
 
 int attention_chunk();
 int sample_small_cap();

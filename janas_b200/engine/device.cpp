@@ -1,5 +1,7 @@
 #include "device.h"
 
+#include "../csrc/launch.h"
+
 #include <cstring>
 
 namespace jb {
@@ -202,7 +204,11 @@ void Device::upload_pinned(void *dst, const void *src, size_t bytes) {
     Stage *s = nullptr;
     if (last_ >= 0 && ring_[(size_t)last_].host == src) s = &ring_[(size_t)last_];
     if (!s) fail(JB_LLM_EFAIL, "upload_pinned: not the buffer that pinned() gave last");
-    if (bytes) cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream), "copy to the device");
+    // small arrays of whole words by a kernel (see jb_copy_words); what is large goes at the copy engine's pace
+    if (bytes % 4 == 0 && bytes <= (256u << 10) && (uintptr_t)dst % 4 == 0 && bytes > 0)
+        ops::copy_words(*this, src, dst, (long long)(bytes / 4), true);
+    else if (bytes)
+        cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream), "copy to the device");
     cuda_check(cudaEventRecord(s->done, stream), "cudaEventRecord");
     s->used = true;
     h2d_bytes += (long long)bytes;

@@ -91,22 +91,20 @@ PendingDecode *DecodeGraph::begin(const std::vector<int> &slots, const int32_t *
     int32_t *d = (int32_t *)dev_.ptr;
     if (sampled_ && long_way_) e.sampler_scratch();      // allocated before any capture
     if (tokens) {
-        cuda_check(cudaMemcpyAsync(d, h, total_ * 4, cudaMemcpyHostToDevice, dv.stream), "copy to the device");
+        ops::copy_words(dv, h, d, (long long)total_, true);
         dv.h2d_bytes += (long long)total_ * 4;
     } else {
         if (before && before != this)
             cuda_check(cudaMemcpyAsync(d, before->dev_.ptr, (size_t)B * 4, cudaMemcpyDeviceToDevice, dv.stream),
                        "copy on the device");
-        cuda_check(cudaMemcpyAsync(d + B, h + B, (total_ - (size_t)B) * 4, cudaMemcpyHostToDevice, dv.stream),
-                   "copy to the device");
+        ops::copy_words(dv, h + B, d + B, (long long)total_ - B, true);
         dv.h2d_bytes += (long long)(total_ - (size_t)B) * 4;
     }
     if (!exec_) {
         // the first step runs eagerly (it brings every temporary into the pool and is
         // a real step); the capture that follows records without running
         launch(false);
-        cuda_check(cudaMemcpyAsync(out_host_[turn], d, (size_t)B * 4, cudaMemcpyDeviceToHost, dv.stream),
-                   "reading the chosen tokens");
+        ops::copy_words(dv, d, out_host_[turn], B, false);
         cuda_check(cudaEventRecord(events_[turn], dv.stream), "cudaEventRecord");
         dv.sync();
         long long before_n = ops::launches();
@@ -129,8 +127,7 @@ PendingDecode *DecodeGraph::begin(const std::vector<int> &slots, const int32_t *
     } else {
         cuda_check(cudaGraphLaunch(exec_, dv.stream), "cudaGraphLaunch");
         ops::count_launches(kernels);
-        cuda_check(cudaMemcpyAsync(out_host_[turn], d, (size_t)B * 4, cudaMemcpyDeviceToHost, dv.stream),
-                   "reading the chosen tokens");
+        ops::copy_words(dv, d, out_host_[turn], B, false);
         cuda_check(cudaEventRecord(events_[turn], dv.stream), "cudaEventRecord");
     }
     pending_[turn] = PendingDecode();
