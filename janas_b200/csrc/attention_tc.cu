@@ -845,6 +845,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
 //
 // A CTA runs over its chunks with a running (m, l, O) and leaves one partial per
 // head in scratch; attention.cu's merge kernel joins the CTAs' partials.
+constexpr int DQ_THREADS = 192;          // warp 0 loads, warp 1 issues MMAs, 2..5 keys, then values
 constexpr int DQ_N = 16;                 // heads per MMA (N)
 constexpr int DQ_BLK = DQ_N * 128;       // a block of 16 rows of 128 bytes
 // The ring holds units of 32 KB: the keys of a chunk, then its values, then the
@@ -886,7 +887,7 @@ __device__ __forceinline__ float4 load_w4(const void *w, int w_f32, int at)
 
 // GP: the group's heads rounded up to a power of two (the row threads' loops).
 template <int GP>
-__global__ void __launch_bounds__(192)
+__global__ void __launch_bounds__(DQ_THREADS)
 attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v,
@@ -915,13 +916,35 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
         prefetch_tensor_map(&map_v);
         prefetch_tensor_map(&map_q);
     }
-    int kvh = blockIdx.y;
+    // The longest rows' CTAs start first, a row's KV heads next to each other: a long run that starts behind short ones
+    // ends long after everything else (64 sequences of 64 to 2,048 positions, lengths spread evenly over the logarithm:
+    // nine steps of four layers 4,909 -> 4,490 us, all 64 at 2,000 502 -> 484 a step).  The rows' ranks by position are taken anew by every CTA, from what was written long before the
+    // kernel ahead; more rows than threads keep their order.
+    const unsigned place = blockIdx.y * gridDim.x + blockIdx.x;
+    const int kvh = (int)(place % gridDim.y);
     // max_chunks counts the kept first tokens' chunks (kc, one partial each, first among a
     // row's partials) and then the window's, chunks_per_cta to a partial
     int kc = window > 0 && f.keep_first > 0 ? (f.keep_first + AT_KEYS - 1) / AT_KEYS : 0;
     int parts = kc + (max_chunks - kc + chunks_per_cta - 1) / chunks_per_cta;
     int max_parts = parts;             // partials per (row, head) in scratch
-    int lrow = blockIdx.x / parts, part_i = blockIdx.x % parts;
+    int lrow = (int)(place / gridDim.y) / parts, part_i = (int)(place / gridDim.y) % parts;
+    const int n_rows = (int)gridDim.x / parts;
+    if (n_rows > 1 && n_rows <= DQ_THREADS) {
+        int *pos_s = (int *)p_s, *row_s = pos_s + DQ_THREADS, t = threadIdx.x, mine = 0, rank = 0;
+        if (t < n_rows)
+            pos_s[t] = mine = row_pos[row0 + t];
+        __syncthreads();
+        if (t < n_rows) {
+            for (int u = 0; u < n_rows; u++) {
+                int p = pos_s[u];
+                rank += p > mine || (p == mine && u < t);
+            }
+            if (rank == lrow)
+                *row_s = t;
+        }
+        __syncthreads();
+        lrow = *row_s;
+    }
     int q_row = row0 + lrow;
     int q_pos = row_pos[q_row];
     int seq = row_seq[q_row];
@@ -1576,7 +1599,7 @@ static int attn_tc_decode(const void *q, const void *k_cache, const void *v_cach
         static unsigned long long smem_allowed = 0;                                            \
         if (!allow_dynamic_smem(attn_tc_decode_kernel<GP>, DQ_SMEM, smem_allowed))             \
             return JB_ELAUNCH;                                                                 \
-        launch(attn_tc_decode_kernel<GP>, dim3(gx, nkv), 192, DQ_SMEM, st,                     \
+        launch(attn_tc_decode_kernel<GP>, dim3(gx, nkv), DQ_THREADS, DQ_SMEM, st,                     \
                mq, mk, mv, row_pos, row_seq, block_table, bt_stride, part, nh, nkv, G, window, \
                scale, max_chunks, chunks_per_cta, row0, f);                                    \
     } while (0)
