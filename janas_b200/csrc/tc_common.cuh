@@ -256,6 +256,14 @@ __host__ __device__ constexpr uint32_t instr_desc_bf16(int m, int n, bool b_mn_m
            ((uint32_t)(m >> 4) << 24);
 }
 
+// The warp's maximum in one instruction (NaN only if all are NaN, like fmaxf).
+__device__ __forceinline__ float warp_max_redux(float v)
+{
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // 2^x in one instruction (ex2.approx.ftz: relative error about 2^-22; -inf gives 0).
 __device__ __forceinline__ float fast_exp2(float x)
 {
