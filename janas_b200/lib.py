@@ -76,9 +76,9 @@ class GenStatsC(ctypes.Structure):
 
 
 class Piece(ctypes.Structure):
-    _fields_ = [("slot", ctypes.c_int32), ("n", ctypes.c_uint32),
-                ("tokens", ctypes.POINTER(ctypes.c_int32)), ("n_want", ctypes.c_uint32),
-                ("want", ctypes.POINTER(ctypes.c_int32))]
+    # (tokens and want are pointers to int32, held as addresses)
+    _fields_ = [("slot", ctypes.c_int32), ("n", ctypes.c_uint32), ("tokens", ctypes.c_void_p),
+                ("n_want", ctypes.c_uint32), ("want", ctypes.c_void_p)]
 
 
 PART_CALLBACK = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_char_p,

@@ -38,3 +38,21 @@ def test_a_decode_step_wants_a_token_for_every_slot(tokens):
     eng = object.__new__(Engine)            # refused before the library is called
     with pytest.raises(StepError, match="tokens for 2 sequences"):
         eng.decode_begin([0, 1], tokens)
+
+
+@pytest.mark.parametrize("kind", [list, tuple, np.array, torch.tensor])
+def test_packing_of_a_step(kind):
+    """All entries' tokens and wanted places go into one array: every piece has its own, whatever holds them."""
+    import ctypes
+    from janas_b200.engine.engine import StepEntry
+    entries = [(3, kind([5, 6, 7]), [0, 2]), StepEntry(9, kind([2 ** 31 - 1]), ()), (4, kind([8, 1]), kind([1])), (0, [], []),
+               (2, [4.0, Fraction(3)], [1])]
+    pieces, keep, wanted = object.__new__(Engine)._pieces(entries)
+    assert wanted == 4 and len(pieces) == 5
+
+    def at(address, n):
+        return [ctypes.c_int32.from_address(address + 4 * i).value for i in range(n)]
+
+    got = [(p.slot, at(p.tokens, p.n), at(p.want, p.n_want)) for p in pieces]
+    assert got == [(3, [5, 6, 7], [0, 2]), (9, [2 ** 31 - 1], []), (4, [8, 1], [1]), (0, [], []), (2, [4, 3], [1])]
+    assert all(p.tokens and p.want for p in pieces)
