@@ -860,16 +860,16 @@ __global__ void attn_merge_kernel(const float *__restrict__ part,
                                   long long head_major_rows, int keep_first, int plain_sum)
 {
     pdl_trigger();
-    pdl_wait();
     int lrow = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
     int row = row0 + lrow;
-    int pos = row_pos[row];
+    int pos = row_pos[row];          // (the positions were there before the kernel ahead: not after the wait, one trip less)
     int lo = window > 0 && pos + 1 > window ? pos + 1 - window : 0;
     // a partial covers chunks_per_part chunks; max_chunks is the partials' stride
     int n_chunks = (pos / ATT_CHUNK - lo / ATT_CHUNK + chunks_per_part) / chunks_per_part +
                    kept_chunks(window, keep_first);
     const float *base = part + part_at((size_t)lrow, nh, h, max_chunks, 0, hd);
     size_t stride = part_at(0, nh, 0, max_chunks, 1, hd);
+    pdl_wait();
     if (plain_sum) {
         // weights that are not normalized over the keys: the partials' sums, in chunk order
         float acc = 0.0f;
@@ -884,12 +884,16 @@ __global__ void attn_merge_kernel(const float *__restrict__ part,
         return;
     }
     float m = -INFINITY, l = 0.0f, o = 0.0f;
-    // a row with few partials fetches four at a time, one with more sixteen, one
-    // with many thirty-two: most rows need one trip to memory
+    // a row with few partials fetches four at a time, one with more eight, sixteen or
+    // twenty-four, one with many thirty-two: most rows need one trip to memory
     if (n_chunks <= 4) {
         merge_partials<4>(base, stride, 0, n_chunks, d, hd, m, l, o);
+    } else if (n_chunks <= 8) {
+        merge_partials<8>(base, stride, 0, n_chunks, d, hd, m, l, o);
     } else if (n_chunks <= 16) {
         merge_partials<16>(base, stride, 0, n_chunks, d, hd, m, l, o);
+    } else if (n_chunks <= 24) {
+        merge_partials<24>(base, stride, 0, n_chunks, d, hd, m, l, o);
     } else {
         for (int c0 = 0; c0 < n_chunks; c0 += 32)
             merge_partials<32>(base, stride, c0, n_chunks, d, hd, m, l, o);

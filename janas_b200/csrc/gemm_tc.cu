@@ -98,15 +98,26 @@ __device__ __forceinline__ void store_partial(uint32_t taddr, int hgrp, float *_
 {
     constexpr int COLS = MT * BN;
     if constexpr (BN < 32) {
-        float v[16];
-        if (hgrp != 0)
+        // the two warps of a quarter have eight tokens each
+        static_assert(BN == 16 && MT == 1, "two halves of eight");
+        int rows = min(n - n0 - 8 * hgrp, 8);
+        if (rows <= 0)
             return;
-        tc_ld16(taddr, v);
+        uint32_t v[8];
+        tc_ld8_nowait(taddr + 8 * hgrp, v);
+        tc_ld_wait();
         if (f < m) {
+            float *p = dst + (size_t)(n0 + 8 * hgrp) * m + f;
+            if (rows == 8) {
 #pragma unroll
-            for (int j = 0; j < 16; j++)
-                if (n0 + j < n)
-                    dst[(size_t)(n0 + j) * m + f] = v[j];
+                for (int j = 0; j < 8; j++, p += m)
+                    *p = __uint_as_float(v[j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; j++, p += m)
+                    if (j < rows)
+                        *p = __uint_as_float(v[j]);
+            }
         }
     } else {
         uint32_t va[32], vb[32];
@@ -205,9 +216,11 @@ __device__ __forceinline__ void store_swiglu(uint32_t taddr, int hgrp, bf16 *__r
 }
 
 // The same for a tile whose TMEM lanes [0, 64) are gate features and [64, 128) the
-// up features of the same indices: the warps of the upper lanes hand their values
-// to the lower ones through shared memory (xch, 64 rows of BN + 1 floats at the
-// start of the ring, which nothing reads any more).  All eight epilogue warps meet at the
+// up features of the same indices: all values go through shared memory (xch, 128 rows of
+// BN + 1 floats at the start of the ring, which nothing reads any more), so that all 256
+// epilogue threads share the units out, four threads to a feature, and none is made for a
+// token that is not there.  (Two warps made all of them before, one token after the other.
+// With the shorter ends of the plain product: one user's token 2,021 -> 1,966 us.)  All eight epilogue warps meet at the
 // barrier, whether their wait for the accumulator ran out or not.
 template <int BN>
 __device__ __forceinline__ void store_swiglu_half(uint32_t taddr, int q, int lane, int hgrp,
@@ -216,31 +229,27 @@ __device__ __forceinline__ void store_swiglu_half(uint32_t taddr, int q, int lan
                                                   int n0, int n, const GatedUnit &unit)
 {
     const float k = unit.alpha * -1.4426950408889634f;
-    constexpr int LD = BN + 1;
-    float v[16];
-    if (ok && q >= 2) {
-        float *row = xch + ((q - 2) * 32 + lane) * LD;
-        for (int c = 16 * hgrp; c < BN; c += 32) {
-            tc_ld16(taddr + c, v);
+    constexpr int LD = BN + 1, HALF = BN / 2;
+    const int rows = min(n - n0, BN);
+    if (ok) {
+        float *row = xch + (q * 32 + lane) * LD + HALF * hgrp;
 #pragma unroll
-            for (int j = 0; j < 16; j++)
-                row[c + j] = v[j];
+        for (int c = 0; c < HALF; c += 8) {
+            uint32_t v[8];
+            tc_ld8_nowait(taddr + HALF * hgrp + c, v);
+            tc_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                row[c + j] = __uint_as_float(v[j]);
         }
     }
     named_barrier(1, GEMM_THREADS - 64);
-    if (ok && q < 2) {
-        int j0 = q * 32 + lane, f = m0 + j0;
-        const float *row = xch + j0 * LD;
-        for (int c = 16 * hgrp; c < BN; c += 32) {
-            tc_ld16(taddr + c, v);
-            if (f < ff) {
-                bf16 *p = out_act + (size_t)(n0 + c) * ff + f;
-#pragma unroll
-                for (int j = 0; j < 16; j++, p += ff)
-                    if (n0 + c + j < n)
-                        *p = unit_bf16(v[j], row[c + j], k, unit);
-            }
-        }
+    int u = threadIdx.x - 64, j = u % HALF_M, f = m0 + j;
+    if (ok && f < ff) {
+        const float *g = xch + j * LD, *up = g + HALF_M * LD;
+        bf16 *p = out_act + (size_t)n0 * ff + f;
+        for (int t = u / HALF_M; t < rows; t += 4)
+            p[(size_t)t * ff] = unit_bf16(g[t], up[t], k, unit);
     }
 }
 
@@ -356,24 +365,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     } else if (warp == 1 && nkb > 0) {
         // --------------------------------------------------------------- MMAs
         // (the whole warp waits and one lane is elected to issue: see tc_mma4)
+        // In a decode step most of a CTA's stages are there when this loop begins, and what it takes a stage stands
+        // between the activations' arrival and the product's end: the next stage's barrier is looked at under this one's
+        // MMAs, and a stage that is not used again is not reported free.  (With many tokens the MMAs outlast all that.)
         constexpr uint32_t idesc = instr_desc(BN);
         int s = 0;
         uint32_t ph = 0;
+        constexpr bool FEW = MT == 1;
+        bool there = FEW && mbar_test(full0, 0);
         for (int i = 0; i < nkb; i++) {
-            if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph, abort, &g_gemm_tc_error, 2)))
+            if (!__all_sync(0xffffffffu, there) &&
+                !__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph, abort, &g_gemm_tc_error, 2)))
                 break;
+            uint32_t base = smem_u32(smem) + s * Cfg::STAGE_BYTES, free = empty0 + 8 * s;
+            if (++s == STAGES) {
+                s = 0;
+                ph ^= 1;
+            }
+            there = FEW && mbar_test(full0 + 8 * s, ph);
             tc_fence_after();
-            uint32_t base = smem_u32(smem + s * Cfg::STAGE_BYTES);
             uint64_t da = smem_desc(base + MT * W_TILE_BYTES);
             static_assert(BK / 16 == 4, "four MMAs a stage");
 #pragma unroll
             for (int t = 0; t < MT; t++)
                 tc_mma4<2, 2>(tmem + t * BN, smem_desc(base + t * W_TILE_BYTES), da, idesc, i != 0);
-            tc_commit_warp(empty0 + 8 * s);
-            if (++s == STAGES) {
-                s = 0;
-                ph ^= 1;
-            }
+            if (!FEW || i + STAGES < nkb)
+                tc_commit_warp(free);
         }
         tc_commit_warp(accum);
     } else if (warp >= 2) {

@@ -43,6 +43,22 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
+// Whether the phase with this parity has completed, without waiting.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Waits for the phase with this parity to complete.  Gives up when another
 // thread of the CTA has given up (*abort) or after WAIT_CYCLES; then it records
 // `code` in *err (a device word the host reads), raises *abort and returns false.
@@ -134,6 +150,13 @@ __device__ __forceinline__ void tc_commit_warp(uint32_t bar)
 
 // A value that all lanes of the warp have, as one that the compiler knows to be the same in all of them.
 __device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+
+__device__ __forceinline__ void tc_ld8_nowait(uint32_t taddr, uint32_t *r)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+}
 
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, float *v)
 {
