@@ -34,12 +34,6 @@ public:
     // the tiles alone fill the SMs).  It saves the activation kernel of a decode step
     // and of a short prompt (a prompt of 128 tokens: 3.22 -> 3.13 ms).
     static constexpr long long FUSED_UP_TO = 128;
-    // Between the two: from so many tiles (128 gate and 128 up features by up to 256 rows) on.
-    // The one kernel against the two, us: 2,560 to 9,728 at 137 rows 27.4 against 30.2, at 300
-    // 42.7 against 49.8; 2,048 to 6,144 at 137 21.0 against 30.3; 1,024 to 3,072 (24 tiles) at
-    // 137 11.4 against 15.0; 2,560 to 1,216 (10 tiles) at 137 18.8 against 12.6, at 300 (20)
-    // 19.0 against 16.3, at 450 (20) 19.1 against 21.1.
-    static constexpr long long FUSED_TILES = 24;
 
     SwiGLU(const PartSpec &s, DType dt, Device *d) : FeedForward(s, dt, d) {
         hidden_ = s.get_int("hidden_size");
@@ -74,9 +68,8 @@ public:
         long long n = ctx.n_rows;
         Buf act;
         fused_last_ = false;
-        bool tiles = n > FUSED_UP_TO && (inter_ + 127) / 128 * ((n + 255) / 256) >= FUSED_TILES;
         if (ctx.dtype == BF16 &&
-            (n >= FUSED_FROM || tiles || (n <= FUSED_UP_TO && ops::linear_parts(n, 2 * inter_, hidden_) == 1))) {
+            (n >= FUSED_FROM || (n <= FUSED_UP_TO && ops::linear_parts(n, 2 * inter_, hidden_) == 1))) {
             // enough rows, or enough features, to fill the SMs without cutting k:
             // gate, up and the activation in one kernel
             act = ops::linear_swiglu(d, h, ctx.dtype, n, hidden_, w_gate_up_, unit_);

@@ -105,21 +105,6 @@ def test_swiglu_part_bfloat16(rows, hidden, inter, monkeypatch):
     assert bool((err <= 2 ** -7 * want.abs().max(dim=1).values).all())
 
 
-@pytest.mark.parametrize("rows,inter,fused", [(129, 3072, True), (137, 2945, True), (256, 2944, False), (257, 1472, True),
-                                              (257, 1408, False), (511, 3000, True)])
-def test_swiglu_part_of_some_hundred_rows(rows, inter, fused):
-    """129 to 511 rows: one kernel where its tiles are enough, against the plain feed-forward."""
-    from janas_b200.config import PartSpec
-    ffn = build("feed_forward", PartSpec("swiglu", {"hidden_size": 136, "intermediate_size": inter}), torch.bfloat16)
-    w = give(ffn, "mlp", seed=3, dtype=torch.bfloat16)
-    h = torch.randn(rows, 136).bfloat16()
-    got = ffn.forward(context([0], [rows], torch.bfloat16), h.to(DEV)).sum(0).cpu()
-    assert ffn.info()["fused_last"] == fused
-    want = plain.swiglu(h.float(), w, "mlp.", "bfloat16")
-    err = (got - want).abs().max(dim=1).values
-    assert bool((err <= 2 ** -7 * want.abs().max(dim=1).values).all())
-
-
 @pytest.mark.parametrize("window,qk_norm,rope", [(0, True, True), (20, True, True),
                                                  (0, False, True), (0, True, False)])
 def test_attention_part(window, qk_norm, rope):
