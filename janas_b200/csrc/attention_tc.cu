@@ -853,7 +853,7 @@ constexpr int DQ_BLK = DQ_N * 128;       // a block of 16 rows of 128 bytes
 // are filled by the other's work.
 constexpr int DQ_UNITS = 3;
 constexpr int DQ_UNIT = 2 * BLK_BYTES;       // K (or V) of one chunk, 128 values each
-constexpr int DQ_SMEM = 2 * DQ_BLK + 4 * DQ_BLK + DQ_UNITS * DQ_UNIT + 1024 + 1024;
+constexpr int DQ_SMEM = 2 * DQ_BLK + 4 * DQ_BLK + DQ_UNITS * DQ_UNIT + 1024 + 1280;
 
 // What the kernel needs to make q, and the new position's key and value, itself
 // from the q,k,v product's partial sums (qkv != nullptr): then no kernel stands
@@ -908,7 +908,7 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
     uint32_t *tmem_slot = (uint32_t *)(bars + 14);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
     float *red_m = (float *)(tmem_slot + 4);   // two of [4 warps][16 heads]
-    float *red_l = red_m + 8 * DQ_N;
+    float *red_l = red_m + 8 * DQ_N;           // the same
 
     int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -1078,11 +1078,13 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
                 hi.z = (hi.z * sc) * wh.z; hi.w = (hi.w * sc) * wh.w;
             }
             if (!is_v && f.cs != nullptr) {
+                // (spelled out as the compiler takes the rope kernel's: left to it, either product may be the one
+                // that is rounded)
                 float4 a = lo, b = hi;
-                lo = make_float4(a.x * co.x - b.x * si.x, a.y * co.y - b.y * si.y,
-                                 a.z * co.z - b.z * si.z, a.w * co.w - b.w * si.w);
-                hi = make_float4(a.x * si.x + b.x * co.x, a.y * si.y + b.y * co.y,
-                                 a.z * si.z + b.z * co.z, a.w * si.w + b.w * co.w);
+                lo = make_float4(fmaf(a.x, co.x, -__fmul_rn(b.x, si.x)), fmaf(a.y, co.y, -__fmul_rn(b.y, si.y)),
+                                 fmaf(a.z, co.z, -__fmul_rn(b.z, si.z)), fmaf(a.w, co.w, -__fmul_rn(b.w, si.w)));
+                hi = make_float4(fmaf(a.x, si.x, __fmul_rn(b.x, co.x)), fmaf(a.y, si.y, __fmul_rn(b.y, co.y)),
+                                 fmaf(a.z, si.z, __fmul_rn(b.z, co.z)), fmaf(a.w, si.w, __fmul_rn(b.w, co.w)));
             }
             if (is_q) {
                 // where the TMA load would have put it: block of the half, row of the
@@ -1232,8 +1234,8 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
         for (int g = 0; g < GP; g++)
             sb2[g] = sig && g < G ? f.score_bias[kvh * G + g] * 1.4426950408889634f : 0.0f;
         bool ok = true;
-        // running over this CTA's chunks: maximum (every thread keeps all heads'), this thread's key's part of the
-        // sum and its value of O for every head
+        // running over this CTA's chunks: maximum, sum (every thread keeps all heads')
+        // and this thread's value of O for every head
         float m_run[GP], l_run[GP], o_acc[GP], alpha[GP];
 #pragma unroll
         for (int g = 0; g < GP; g++) {
@@ -1259,10 +1261,16 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
         };
         // A chunk is a chain of steps that nothing else of this CTA hides, and the CTAs of an SM are two: what it takes
         // bounds the kernel.  So the heads are taken side by side (no branch between one head's steps and the next's), a
-        // warp's maximum is one instruction, the sum of the weights is kept by key and added up once at the end, and one
-        // barrier a chunk passes the warps' maxima on.  One chunk took 3,700 cycles with a reduction by shuffles per
-        // head, of maximum and of sum, and two barriers; now 1,300, and the kernel waits for its keys (8 sequences at 2,048: 1,088
-        // chunks of 64 KB in 11.7 us).
+        // warp's maximum is one instruction, the sums of the weights are added up when the weights are on their way, and
+        // one barrier a chunk passes the warps' maxima of this chunk and their sums of the last one on.  A chunk took 3,700
+        // cycles with the heads' reductions one after the other and two barriers; now about 1,400, and the kernel waits for
+        // its keys (8 sequences at 2,048: 1,088 chunks of 64 KB in 11.7 us).
+        auto take_l = [&](int it) {
+            const float *red = red_l + (it & 1) * 4 * DQ_N;
+#pragma unroll
+            for (int g = 0; g < GP; g++)
+                l_run[g] = l_run[g] * alpha[g] + (red[g] + red[DQ_N + g] + red[2 * DQ_N + g] + red[3 * DQ_N + g]);
+        };
         for (int it = 0; it < n_chunks; it++) {
             int c = c_first + it;
             int t = c * AT_KEYS + r;
@@ -1305,8 +1313,10 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
             named_barrier(1, AT_ROWS);
             // the chunk before this one is taken into O with ITS alpha, before alpha
             // is overwritten below
-            if (it > 0)
+            if (it > 0) {
+                take_l(it - 1);
                 take_o(it - 1);
+            }
 #pragma unroll
             for (int g = 0; g < GP; g++)
                 m[g] = fmaxf(fmaxf(red[g], red[DQ_N + g]), fmaxf(red[2 * DQ_N + g], red[3 * DQ_N + g]));
@@ -1324,9 +1334,6 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
                     sc[g] = sc[g] == -INFINITY ? 0.0f : e;
                 }
             }
-#pragma unroll
-            for (int g = 0; g < GP; g++)
-                l_run[g] = l_run[g] * alpha[g] + sc[g];
             // P[head][key] in bfloat16, buffer it % 2 (chunk it - 2's P V has been waited
             // for): block r / 64, row g, 16-byte chunk (r % 64) / 8
             {
@@ -1340,20 +1347,17 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
             fence_async_smem();
             tc_fence_before();
             mbar_arrive(bar(9 + (it & 1)));
-        }
-        // the keys' parts of the sums, over the warp and then over the warps
-#pragma unroll
-        for (int g = 0; g < GP; g++)
-            l_run[g] = warp_sum(l_run[g]);
-        if (lane == 0) {
 #pragma unroll
             for (int g = 0; g < GP; g++)
-                red_l[qw * DQ_N + g] = l_run[g];
+                sc[g] = warp_sum(sc[g]);
+            if (lane == 0) {
+#pragma unroll
+                for (int g = 0; g < GP; g++)
+                    red_l[((it & 1) * 4 + qw) * DQ_N + g] = sc[g];
+            }
         }
         named_barrier(1, AT_ROWS);
-#pragma unroll
-        for (int g = 0; g < GP; g++)
-            l_run[g] = red_l[g] + red_l[DQ_N + g] + red_l[2 * DQ_N + g] + red_l[3 * DQ_N + g];
+        take_l(n_chunks - 1);
         take_o(n_chunks - 1);
         // one partial for this CTA's run of chunks
         if (ok) {
