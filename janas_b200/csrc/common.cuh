@@ -157,7 +157,14 @@ __device__ __forceinline__ void split2(f32x2 v, float &lo, float &hi)
 // pdl_wait() blocks until the kernel before this one has completed and its
 // writes are visible.  What a kernel does before pdl_wait() must not touch
 // anything an earlier kernel writes or reads-and-frees: only its own shared and
-// tensor memory and the (immutable) weights.
+// tensor memory, the (immutable) weights and a step's inputs (positions, sequence
+// indices, slots, block tables, query blocks).  Those are written by copies that stand
+// ahead of every kernel that reads them and that no later kernel starts beside: a copy
+// engine's copy, which the kernel behind it waits for as a whole, or convert.cu's
+// copy_words_kernel, which never triggers and whose threads end only after a
+// device-wide fence behind their stores.  So a kernel that reads them, however early it
+// starts, starts after they can be read.  A kernel of a step that wrote such an input
+// for a later kernel of the step would break this.
 // A kernel argument that an earlier kernel writes and that is read right after pdl_wait() should not be
 // const __restrict__: the compiler takes such memory for read-only and may move the load ahead of the
 // wait.

@@ -26,8 +26,9 @@ __global__ void convert_kernel(const S *__restrict__ src, D *__restrict__ dst, l
 }
 
 // dst[i] = src[i], a word a thread, either side pinned host memory.  The words of the host are on their way before the
-// kernel ahead has ended (src_early: nothing on the stream writes src).  Never allows the kernel behind it to start early:
-// kernels read a step's positions and tables ahead of their own waits.
+// kernel ahead has ended (src_early: nothing on the stream writes src).  Never allows the kernel behind it to start early,
+// and no thread ends before its word can be read by the whole device: kernels read a step's positions and tables ahead of
+// their own waits (see common.cuh: pdl_wait), and only the kernel right behind this one could wait for its end.
 __global__ void __launch_bounds__(256)
 copy_words_kernel(const uint32_t *src, uint32_t *dst, int n, int src_early)
 {
@@ -40,6 +41,7 @@ copy_words_kernel(const uint32_t *src, uint32_t *dst, int n, int src_early)
         v = __ldcv(src + i);
     if (i < n)
         __stcg(dst + i, v);
+    __threadfence();
 }
 
 }  // namespace

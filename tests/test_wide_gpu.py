@@ -207,6 +207,43 @@ def test_bfloat16_under_other_cuts(runs):
     print(f"bfloat16, other cuts against whole: {worst:.3e}")
 
 
+# ------------------------------------------------------------------ steps one behind the other
+def test_steps_launched_one_behind_the_other_see_their_own_inputs():
+    """Eager steps whose positions, sequence indices and block tables alternate in the same pooled buffer, launched
+    back to back: kernels read them ahead of their own waits.  The same bits as with every step waited for."""
+    from janas_b200.engine import StepEntry
+    rng = np.random.default_rng(5)
+    lens = [700, 20, 301, 64, 129, 511]
+    prompts = [rng.integers(0, WIDE["vocab_size"], size=n).tolist() for n in lens]
+    extra = rng.integers(0, WIDE["vocab_size"], size=(12, len(lens))).tolist()
+
+    def go(wait):
+        eng = engine("bfloat16", max_tokens=len(lens) * 768, max_seqs=len(lens))
+        slots = [eng.new_sequence() for _ in lens]
+        out = []
+        for s, p in zip(slots, prompts):
+            eng.step_numpy([StepEntry(s, p)])
+            if wait:
+                torch.cuda.synchronize()
+        for i, toks in enumerate(extra):
+            order = [(j * 5 + i) % len(lens) for j in range(3 if i % 2 else 2)]
+            last = i == len(extra) - 1
+            if last:
+                order = range(len(lens))
+            got = eng.step_numpy([StepEntry(slots[j], [toks[j]], [0] if last else []) for j in order])
+            if wait:
+                torch.cuda.synchronize()
+            if got is not None:
+                out.append(got)
+        eng.check()
+        eng.close()
+        return np.concatenate(out)
+
+    want = go(True)
+    for _ in range(3):
+        assert np.array_equal(go(False), want)
+
+
 # ------------------------------------------------------------------ the products' tiles
 @pytest.mark.parametrize("tile", [128, 160, 192, 224, 256])
 def test_every_tile_width_of_the_many_token_product(tile):
