@@ -1,9 +1,10 @@
 // out[n, m] = A[n, k] . W[m, k]^T in float32 on the fifth-generation tensor cores.
 //
-// A float is the exact sum of three bfloat16 (24 bits of mantissa in three times eight, each rest rounded to
-// nearest: hi, mid, lo), so the product of two floats is nine products of bfloat16, each exact in float32.  The six
-// largest are added up; the three left out are below 2^-26 of the product.  They are tcgen05 MMAs, 128 features by
-// tokens by 16 of k, with float32 accumulators in tensor memory.
+// A float times 2^24 is the exact sum of three bfloat16 (24 bits of mantissa in three times eight, each rest rounded to
+// nearest: hi, mid, lo; the factor keeps the last part of the smallest float above the smallest normal bfloat16, which
+// has the exponents of a float), so the product of two floats is nine products of bfloat16, each exact in float32.  The
+// six largest are added up; the three left out are below 2^-26 of the product.  They are tcgen05 MMAs, 128 features by
+// tokens by 16 of k, with float32 accumulators in tensor memory.  A segment's sum is taken times 2^-48 at its end.
 //
 // Every output value is computed by one fixed recipe, whatever n is, so that a row's result is the same bits
 // however the tokens are cut into steps: k is cut into blocks of 64 at fixed places; a block's accumulator takes the
@@ -25,10 +26,11 @@
 //   tokens 8:    6144 x 2560  16.9 (20.6)  2560 x 4096  14.4 (14.6)  19456 x 2560  44.1 (50.7)  2560 x 9728  23.2 (28.5)
 //   tokens 64:   6144 x 2560  22.0 (65.4)  2560 x 4096  18.7 (45.6)  19456 x 2560  58.1 (207)   2560 x 9728  30.0 (117)
 //   tokens 300:  6144 x 2560  57.0 (271)   2560 x 4096  45.6 (172)   19456 x 2560  171 (724)    2560 x 9728  83.4 (414)
-// The error against 64 bits is 1.0e-7 to 1.3e-7 of the result for normal numbers (2.9e-7 to 3.0e-7).
+// The error against 64 bits is 1.0e-7 to 1.3e-7 of the result (2.9e-7 to 3.0e-7), also where all of a token or of a
+// feature is small.
 //
-// A sum that is not finite is taken again from the floats by plain multiply-adds (an infinity has no parts, and a
-// finite sum of finite products never gets there unless it overflows on the way).
+// A sum that is not finite is taken again from the floats by plain multiply-adds: an infinity has no parts, and neither
+// has a float from 2^104 up; a finite sum of finite products gets there from 2^80 up, or where it overflows on the way.
 //
 // The reference computes y = W x with rows of W as output features (src/llm/model_load.c:452); its products are
 // over quantized blocks and are not reproduced.
@@ -182,7 +184,10 @@ __device__ __forceinline__ void tc_ld16_nowait(uint32_t taddr, uint32_t *r)
         : "r"(taddr));
 }
 
-// two floats' parts, the first in the lower halves
+// Both operands' factor, and what takes both out of a sum again.
+constexpr float F_UP = 16777216.0f, F_DOWN = 1.0f / F_UP / F_UP;
+
+// The parts of two floats times F_UP, the first in the lower halves.
 __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi)
 {
     uint32_t d;
@@ -191,12 +196,16 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi)
 }
 __device__ __forceinline__ void parts_of(float x, float y, uint32_t &p0, uint32_t &p1, uint32_t &p2)
 {
+    const f32x2 minus = pair2(-1.0f, -1.0f);
+    f32x2 v = mul2(pair2(x, y), pair2(F_UP, F_UP));
+    auto rest = [&](uint32_t p) { return fma2(pair2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)), minus, v); };
+    split2(v, x, y);
     p0 = bf16_pair(x, y);
-    x -= __uint_as_float(p0 << 16);
-    y -= __uint_as_float(p0 & 0xffff0000u);
+    v = rest(p0);
+    split2(v, x, y);
     p1 = bf16_pair(x, y);
-    x -= __uint_as_float(p1 << 16);
-    y -= __uint_as_float(p1 & 0xffff0000u);
+    v = rest(p1);
+    split2(v, x, y);
     p2 = bf16_pair(x, y);
 }
 
@@ -575,10 +584,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 for (int j = 0; j < 8; j++, to += step)
                     if (c + j < rows) {
                         float v = sum[c + j];
-                        if (fabsf(v) <= 3.402823466e38f)
+                        if (fabsf(v) <= 3.402823466e38f) {
+                            v *= F_DOWN;
                             *to = add ? had[j] + v : v;
-                        else
+                        } else {
                             bad[(c + j) / 32] |= 1u << ((c + j) % 32);
+                        }
                     }
             }
 #pragma unroll

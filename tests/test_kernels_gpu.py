@@ -198,6 +198,22 @@ def test_gemm_f32_parts(m, k):
     assert ops().gemm_tc_error() == 0
 
 
+@pytest.mark.parametrize("n", [7, 40])
+@pytest.mark.parametrize("up_a,up_w", [(-100, 0), (-113, 0), (-120, 0), (-126, 0), (0, -113), (0, -126), (-63, -63), (40, 30)])
+def test_gemm_f32_parts_of_small_floats(n, up_a, up_w):
+    """All of the tokens, or of the weights, are small: the parts still hold the floats.  The bound is the one of
+    test_gemm_f32_parts, and 2^-149 for each sum of a segment where the result has no more bits than that; the error as
+    a whole is no larger than the plain kernel's."""
+    k, m = 1100, 600
+    a, w = rnd(n, k) * 2.0 ** up_a, rnd(m, k, seed=3) * 2.0 ** up_w
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    got = ops().linear(a.to(DEV), w.to(DEV))[0].cpu().double()
+    plain_way = ops().linear(a.to(DEV), w.to(DEV), force_simt=True)[0].cpu().double()
+    bound = (1 + 17 * 5 + 2 * -(-k // 64)) * 2.0 ** -24 * size + 8 * 2.0 ** -149
+    assert ((got - want).abs() <= bound).all()
+    assert (got - want).norm() <= (plain_way - want).norm()
+
+
 @pytest.mark.parametrize("n", [5, 70])
 def test_gemm_f32_parts_not_finite(n):
     """Infinities, NaN and floats too large for a part, in single rows and features: the products of the plain kernel
