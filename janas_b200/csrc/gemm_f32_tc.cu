@@ -209,17 +209,62 @@ __device__ __forceinline__ void parts_of(float x, float y, uint32_t &p0, uint32_
     p2 = bf16_pair(x, y);
 }
 
-// A segment's sum for one token and feature, by multiply-adds: even and odd k in a chain each.
-__device__ __forceinline__ float plain_segment(const float *a, const float *w, int k0, int k1)
+// A segment (k0 <= k < k1, multiples of four) of four tokens for a lane's feature, where sums were not finite: by
+// multiply-adds, even and odd k in a chain each.  a: the first token, rows of k floats, `last` the last that there is; bad:
+// the sums to make, a bit a token; to, step: where they go, added to what is there or not.  A token's NaN makes all of its
+// sums one, and a run that went wrong has little else: looked for first, without the weights, of which every lane reads a
+// row of its own.  One B200, us, 320 rows of 12288 x 2048 (one segment; finite 120, gemm_simt.cu 393): all NaN 3,020, all
+// infinite 8,700; 300 of 2560 x 9728 (98, 433) 1,190 and 3,170; 8 of those (46, 47) 94 and 270.  A token and a feature
+// at a time, as it was: 46,100, 17,500 and 1,040.
+__device__ __noinline__ void plain_sums(const float *a, int k, int last, int a_vec, const float *w, int k0, int k1,
+                                        uint32_t bad, float *to, size_t step, bool add)
 {
-    float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll 1
-    for (int i = k0; i < k1; i += 2) {
-        s0 = fmaf(a[i], w[i], s0);
-        if (i + 1 < k1)
-            s1 = fmaf(a[i + 1], w[i + 1], s1);
+    const float *row[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+        row[t] = a + (size_t)min(t, last) * k;
+    bool nan[4] = {};
+    if (a_vec) {
+#pragma unroll 2
+        for (int i = k0; i < k1; i += 4)
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const float4 v = load4(row[t] + i);
+                nan[t] |= isnan(v.x) | isnan(v.y) | isnan(v.z) | isnan(v.w);
+            }
+    } else {
+#pragma unroll 4
+        for (int i = k0; i < k1; i++)
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                nan[t] |= isnan(row[t][i]);
     }
-    return s0 + s1;
+    float s0[4], s1[4];
+    bool sums = false;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        s0[t] = s1[t] = nan[t] ? __int_as_float(0x7fffffff) : 0.0f;
+        sums |= !nan[t] && (bad >> t & 1);
+    }
+    if (sums) {
+#pragma unroll 1
+        for (int i = k0; i < k1; i += 4) {
+            const float4 u = load4(w + i);
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const float *p = row[t] + i;
+                const float4 v = a_vec ? load4(p) : make_float4(p[0], p[1], p[2], p[3]);
+                s0[t] = fmaf(v.x, u.x, s0[t]);
+                s1[t] = fmaf(v.y, u.y, s1[t]);
+                s0[t] = fmaf(v.z, u.z, s0[t]);
+                s1[t] = fmaf(v.w, u.w, s1[t]);
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 4; t++, to += step)
+        if (bad >> t & 1)
+            *to = add ? *to + (s0[t] + s1[t]) : s0[t] + s1[t];
 }
 
 template <int BN>
@@ -595,11 +640,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
             for (int w = 0; w < (COLS + 31) / 32; w++)
                 while (bad[w]) {
-                    int c = w * 32 + __ffs(bad[w]) - 1;
-                    bad[w] &= bad[w] - 1;
-                    float v = plain_segment(A + (size_t)(n0 + c) * work.k, W + (size_t)f * work.k,
-                                            cur.seg * work.seg_blocks * F_BK, min(work.k, (cur.seg + 1) * work.seg_blocks * F_BK));
-                    p[(size_t)c * step] = add ? p[(size_t)c * step] + v : v;
+                    const int g = (__ffs(bad[w]) - 1) & ~3, c = w * 32 + g;
+                    plain_sums(A + (size_t)(n0 + c) * work.k, work.k, rows - c - 1, a_vec, W + (size_t)f * work.k,
+                               cur.seg * work.seg_blocks * F_BK, min(work.k, (cur.seg + 1) * work.seg_blocks * F_BK),
+                               bad[w] >> g & 15, p + (size_t)c * step, step, add);
+                    bad[w] &= ~(15u << g);
                 }
         }
     }
@@ -751,10 +796,11 @@ using namespace jb;
 
 // Whether this kernel takes a product; says nothing about n, so that a row's bits do not depend on the batch.  Smaller
 // weights are left to the plain kernel: at 8 tokens 512 x 1024 takes 7.3 us (7.8 there) and 1000 x 1028 7.5 (7.8), but
-// 512 x 512 7.2 (6.7), 2560 x 512 7.4 (6.8) and 256 x 256 5.4 (3.9).
+// 512 x 512 7.2 (6.7), 2560 x 512 7.4 (6.8) and 256 x 256 5.4 (3.9).  Longer rows too: a tile whose sums are all infinite
+// takes the epilogue some 4,500 cycles a k (23 ms at 9,728), and the others' waits end after 2 * 10^9.
 extern "C" int jb_gemm_f32_tc_ok(const void *W, int m, int k)
 {
-    return m >= 512 && k >= 1024 && k % 4 == 0 && (uintptr_t)W % 16 == 0 && k <= 1 << 20;
+    return m >= 512 && k >= 1024 && k % 4 == 0 && (uintptr_t)W % 16 == 0 && k <= 1 << 17;
 }
 
 // Floats of scratch (0: none), and kernels that a call launches.

@@ -232,6 +232,25 @@ def test_gemm_f32_parts_not_finite(n):
     assert ((got - want)[ok].abs() <= 2e-6 * (b.double().abs() @ v.double().abs().T)[ok]).all()
 
 
+@pytest.mark.parametrize("m,k,n", [(12288, 2048, 320), (1100, 2560, 21), (600, 1028, 70)])
+@pytest.mark.parametrize("what", [math.nan, math.inf, 3.0e38])
+def test_gemm_f32_parts_nothing_finite(m, k, n, what):
+    """A value in every token that makes all sums but one feature's infinite or NaN, in segments of any length: the
+    plain kernel's answers, and no wait runs out meanwhile."""
+    a, w = rnd(n, k).to(DEV), rnd(m, k, seed=3).to(DEV)
+    at = torch.arange(n, device=DEV) * 37 % k
+    a[torch.arange(n, device=DEV), at] = what
+    w[5] = 0
+    got, want = ops().linear(a, w)[0], ops().linear(a, w, force_simt=True)[0]
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got[want.isinf()], want[want.isinf()])
+    ok = want.isfinite()
+    size = a.double().abs() @ w.double().abs().T
+    assert ((got.double() - want.double())[ok].abs() <= 2 * k * 2.0 ** -24 * size[ok]).all()
+    assert torch.equal(ops().linear(a[:9].contiguous(), w)[0].nan_to_num(7.0), got[:9].nan_to_num(7.0))
+    assert ops().gemm_tc_error() == 0
+
+
 @pytest.mark.parametrize("odt", DTYPES)
 def test_swiglu(odt):
     n, ff = 7, 300

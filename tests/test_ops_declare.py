@@ -60,3 +60,12 @@ def test_small_headers():
                                             ctypes.c_void_p, ctypes.c_int32]
     with pytest.raises(KeyError):
         ops.declare(_Lib(), "int jb_bad(short s);")      # a type the table does not know
+
+
+def test_which_float_products_go_in_parts():
+    """By the weight alone: features and k from a size on, rows that TMA takes, and no k so long that a tile without a
+    finite sum could outlast the kernel's waits."""
+    ok = ops.lib().jb_gemm_f32_tc_ok
+    assert ok(0, 512, 1024) and ok(0, 513, 1028) and ok(0, 151936, 2560) and ok(0, 512, 1 << 17)
+    assert not ok(0, 511, 1024) and not ok(0, 512, 1020) and not ok(0, 512, 1026) and not ok(4, 512, 1024)
+    assert not ok(0, 512, (1 << 17) + 4)
