@@ -756,24 +756,50 @@ static int f32_seg_blocks(int m, int k)
     return len < 4 ? 4 : len;
 }
 
+// How the next rows of a call are taken: `rows` of them, all at once where the scratch is enough for that.  A row's bits
+// do not depend on it.
 struct F32Plan {
-    int bn, whole, rest, seg_blocks, segments;
+    int rows, bn, seg_blocks, segments;
+    long long whole, rest;              // tiles taken over all of k, and shared out by segments
     long long plane_floats, part_floats;
+    long long floats() const { return plane_floats + part_floats; }
 };
 
-static F32Plan f32_plan(int n, int m, int k)
+static F32Plan f32_pass(int rows, int m, int k, bool share)
 {
     F32Plan p;
-    p.bn = f32_tile(n);
+    p.rows = rows;
+    p.bn = f32_tile(rows);
     p.seg_blocks = f32_seg_blocks(m, k);
     p.segments = ((k + F_BK - 1) / F_BK + p.seg_blocks - 1) / p.seg_blocks;
-    long long tiles = ((long long)m + F_M - 1) / F_M * ((n + p.bn - 1) / p.bn), places = sm_count();
-    // tiles that fill every SM are taken whole; the rest is shared out by segments
-    p.whole = (int)(p.segments == 1 ? tiles : tiles / places * places);
-    p.rest = (int)(tiles - p.whole);
-    p.part_floats = (long long)p.rest * p.segments * p.bn * F_M;
-    p.plane_floats = p.bn > 32 ? ((3ll * n * ((k + 7) / 8 * 8) + 1) / 2 + 63) / 64 * 64 : 0;
+    long long tiles = ((long long)m + F_M - 1) / F_M * (((long long)rows + p.bn - 1) / p.bn), places = sm_count();
+    // tiles that fill every SM are taken whole; the rest is shared out by segments where that ends earlier
+    p.rest = tiles % places;
+    if (!share || (p.rest * p.segments + places - 1) / places >= p.segments)
+        p.rest = 0;
+    p.whole = tiles - p.rest;
+    p.part_floats = p.rest * p.segments * p.bn * F_M;
+    p.plane_floats = p.bn > 32 ? (3ll * rows * ((k + 7) / 8 * 8) / 2 + 63) / 64 * 64 : 0;
     return p;
+}
+
+// The scratch that a call asks for at most.  Planes (6 bytes a value) and shared segments of all rows at once would take
+// 184 MB for 2,048 rows of 2560 x 9728; two passes of 1,024 rows take 65 MB and, by rounds of tiles, the same time.
+constexpr long long F32_SCRATCH = 18ll << 20;           // floats
+
+// The next pass of n rows with `have` floats of scratch: equal passes, as few as fit; up to 32 rows need none.
+static F32Plan f32_plan(int n, int m, int k, long long have)
+{
+    for (int passes = 1;; passes++) {
+        int rows = passes == 1 ? n : (int)(((long long)n + passes - 1) / passes + 31) / 32 * 32;
+        if (rows > n)
+            rows = n;
+        F32Plan p = f32_pass(rows, m, k, true);
+        if (p.floats() <= have)
+            return p;
+        if (rows <= 32)
+            return f32_pass(rows, m, k, false);
+    }
 }
 
 template <int BN>
@@ -803,31 +829,33 @@ extern "C" int jb_gemm_f32_tc_ok(const void *W, int m, int k)
     return m >= 512 && k >= 1024 && k % 4 == 0 && (uintptr_t)W % 16 == 0 && k <= 1 << 17;
 }
 
-// Floats of scratch (0: none), and kernels that a call launches.
+// Floats of scratch that a call asks for (0: none; it makes do with less, or with none, at some cost in time), and kernels
+// that it launches with `have` of them.
 extern "C" long long jb_gemm_f32_tc_scratch(int n, int m, int k)
 {
-    if (n <= 0 || m <= 0 || k <= 0)
-        return 0;
-    F32Plan p = f32_plan(n, m, k);
-    return p.plane_floats + p.part_floats;
+    long long most = 0;
+    for (int r0 = 0; r0 < n && m > 0 && k > 0;) {
+        F32Plan p = f32_plan(n - r0, m, k, F32_SCRATCH);
+        most = p.floats() > most ? p.floats() : most;
+        r0 += p.rows;
+    }
+    return most;
 }
-extern "C" int jb_gemm_f32_tc_launches(int n, int m, int k)
+extern "C" int jb_gemm_f32_tc_launches(int n, int m, int k, long long have)
 {
-    F32Plan p = f32_plan(n, m, k);
-    return 1 + (p.plane_floats > 0) + (p.rest > 0);
+    int kernels = 0;
+    for (int r0 = 0; r0 < n && m > 0 && k > 0;) {
+        F32Plan p = f32_plan(n - r0, m, k, have);
+        kernels += 1 + (p.plane_floats > 0) + (p.rest > 0);
+        r0 += p.rows;
+    }
+    return kernels;
 }
 
-// scratch: jb_gemm_f32_tc_scratch(n, m, k) floats, 16-byte aligned.  early: as jb_gemm_simt.
-extern "C" int jb_gemm_f32_tc(const void *A, const void *W, float *out, int n, int m, int k, float *scratch, int early,
-                              cudaStream_t st)
+static int f32_run(const F32Plan &p, const float *A, const float *W, float *out, int m, int k, float *scratch, int early,
+                   cudaStream_t st)
 {
-    if (n <= 0 || m <= 0)
-        return JB_OK;
-    if (!jb_gemm_f32_tc_ok(W, m, k) || (uintptr_t)A % 4 || (uintptr_t)out % 4)
-        return JB_EINVAL;
-    F32Plan p = f32_plan(n, m, k);
-    if (p.plane_floats + p.part_floats > 0 && (scratch == nullptr || (uintptr_t)scratch % 16))
-        return JB_EINVAL;
+    const int n = p.rows;
     F32Work work;
     work.n = n;
     work.m = m;
@@ -836,27 +864,26 @@ extern "C" int jb_gemm_f32_tc(const void *A, const void *W, float *out, int n, i
     work.segments = p.segments;
     work.seg_blocks = p.seg_blocks;
     work.blocks = (k + F_BK - 1) / F_BK;
-    work.whole = p.whole;
-    if ((long long)p.whole + (long long)p.rest * p.segments > 0x7fffffffll || 3ll * n > 0x7fffffffll ||
-        ((long long)p.rest * p.bn * (F_M / 4) + 255) / 256 > 0x7fffffffll)
+    if (p.whole + p.rest * p.segments > 0x7fffffffll || 3ll * n > 0x7fffffffll)
         return JB_EINVAL;
-    work.units = p.whole + p.rest * p.segments;
+    work.whole = (int)p.whole;
+    work.units = (int)(p.whole + p.rest * p.segments);
     const int a_vec = (uintptr_t)A % 16 == 0, kp = (k + 7) / 8 * 8;
     CUtensorMap map_w, map_a;
     if (!tensor_map_2d(W, m, k, F_M, BOX_K, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, &map_w))
         return JB_EINVAL;
     map_a = map_w;
-    float *part = scratch + p.plane_floats;
+    float *part = p.part_floats > 0 ? scratch + p.plane_floats : nullptr;
     if (p.plane_floats > 0) {
         if (!tensor_map_2d(scratch, 3 * n, kp, p.bn, F_BK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, &map_a))
             return JB_EINVAL;
-        launch(f32_parts_kernel, (unsigned)(((size_t)n * (kp / 4) + 255) / 256), 256, 0, st, (const float *)A,
-               (bf16 *)scratch, n, k, kp, a_vec);
+        launch(f32_parts_kernel, (unsigned)(((size_t)n * (kp / 4) + 255) / 256), 256, 0, st, A, (bf16 *)scratch, n, k, kp,
+               a_vec);
         if (cudaGetLastError() != cudaSuccess)
             return JB_ELAUNCH;
     }
     int rc;
-#define JB_FP(B) rc = f32_launch<B>(map_w, map_a, (const float *)A, (const float *)W, out, part, work, a_vec, early, st)
+#define JB_FP(B) rc = f32_launch<B>(map_w, map_a, A, W, out, part, work, a_vec, early, st)
     switch (p.bn) {
     case 16: JB_FP(16); break;
     case 32: JB_FP(32); break;
@@ -868,9 +895,29 @@ extern "C" int jb_gemm_f32_tc(const void *A, const void *W, float *out, int n, i
 #undef JB_FP
     if (rc != JB_OK || p.rest == 0)
         return rc;
-    launch(f32_join_kernel, (unsigned)(((size_t)p.rest * p.bn * (F_M / 4) + 255) / 256), 256, 0, st,
-           (const float *)part, out, n, m, work.n_tiles, p.whole, work.segments, p.bn);
+    launch(f32_join_kernel, (unsigned)(((size_t)p.rest * p.bn * (F_M / 4) + 255) / 256), 256, 0, st, (const float *)part, out,
+           n, m, work.n_tiles, work.whole, work.segments, p.bn);
     return launch_status();
+}
+
+// scratch: `have` floats, 16-byte aligned; jb_gemm_f32_tc_scratch says how many are worth having, and the results do not
+// depend on it.  early: as jb_gemm_simt.
+extern "C" int jb_gemm_f32_tc(const void *A, const void *W, float *out, int n, int m, int k, float *scratch,
+                              long long have, int early, cudaStream_t st)
+{
+    if (n <= 0 || m <= 0)
+        return JB_OK;
+    if (!jb_gemm_f32_tc_ok(W, m, k) || (uintptr_t)A % 4 || (uintptr_t)out % 4 || (uintptr_t)scratch % 16)
+        return JB_EINVAL;
+    if (scratch == nullptr || have < 0)
+        have = 0;
+    int rc = JB_OK;
+    for (int r0 = 0; r0 < n && rc == JB_OK;) {
+        F32Plan p = f32_plan(n - r0, m, k, have);
+        rc = f32_run(p, (const float *)A + (size_t)r0 * k, (const float *)W, out + (size_t)r0 * m, m, k, scratch, early, st);
+        r0 += p.rows;
+    }
+    return rc;
 }
 
 extern "C" int jb_gemm_f32_tc_error(void)

@@ -308,9 +308,9 @@ int jb_gemm_simt(const void *A, int a_dt, const void *W, int w_dt, float *out, i
                  float *scratch, int early, cudaStream_t st);
 int jb_gemm_f32_tc_ok(const void *W, int m, int k);
 long long jb_gemm_f32_tc_scratch(int n, int m, int k);
-int jb_gemm_f32_tc_launches(int n, int m, int k);
+int jb_gemm_f32_tc_launches(int n, int m, int k, long long have);
 int jb_gemm_f32_tc(const void *A, const void *W, float *out, int n, int m, int k, float *scratch,
-                   int early, cudaStream_t st);
+                   long long have, int early, cudaStream_t st);
 int jb_gemm_f32_tc_error(void);
 int jb_gemm_tc_ok(const void *A, const void *W, int n, int m, int k);
 int jb_gemm_tc_splits(int n, int m, int k);

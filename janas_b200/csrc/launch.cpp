@@ -606,18 +606,35 @@ int linear_parts(long long n, long long m, long long k) {
     return jb_gemm_tc_splits((int)n, (int)m, (int)k);
 }
 
+// Scratch of a product of floats in parts, in one of two sizes, so that all products of a step and steps of any row count
+// take turns with one block (72 MiB: the most that jb_gemm_f32_tc_scratch asks for).  The kernel makes do with less, so a
+// device that has no room for it is no error; the next calls of this device ask for no more than it had.
+static Buf parts_scratch(Device &d, long long floats) {
+    const size_t small = 8u << 20, large = 72u << 20;
+    for (size_t size : {(size_t)floats * 4 > small ? large : small, small}) {
+        if (floats <= 0 || size > d.parts_scratch_limit) continue;
+        Buf b = d.pool.get_if_room(size);
+        if (b) return b;
+        d.parts_scratch_limit = size - 1;
+    }
+    return Buf();
+}
+
 // out = a . w^T whole: floats by the tensor cores in parts where that kernel takes the weight's shape (whatever the
 // rows are, so that a row's bits do not depend on the batch), anything else by plain multiply-adds
 static void plain_product(Device &d, const void *a, DType a_dt, const void *w, DType w_dt, float *out, int n, int m,
                           int k, bool force_simt, const char *what) {
-    bool parts = !force_simt && a_dt == F32 && w_dt == F32 && jb_gemm_f32_tc_ok(w, m, k) != 0;
-    long long need = parts ? jb_gemm_f32_tc_scratch(n, m, k) : jb_gemm_simt_scratch(n, m, k);
+    if (!force_simt && a_dt == F32 && w_dt == F32 && jb_gemm_f32_tc_ok(w, m, k) != 0) {
+        Buf scratch = parts_scratch(d, jb_gemm_f32_tc_scratch(n, m, k));
+        long long have = (long long)(scratch.bytes / 4);
+        check(jb_gemm_f32_tc(a, w, out, n, m, k, scratch.as<float>(), have, 1, d.stream), what,
+              jb_gemm_f32_tc_launches(n, m, k, have));
+        return;
+    }
+    long long need = jb_gemm_simt_scratch(n, m, k);
     Buf scratch;
     if (need > 0) scratch = d.pool.get((size_t)need * 4);
-    if (parts)
-        check(jb_gemm_f32_tc(a, w, out, n, m, k, scratch.as<float>(), 1, d.stream), what, jb_gemm_f32_tc_launches(n, m, k));
-    else
-        check(jb_gemm_simt(a, a_dt, w, w_dt, out, n, m, k, scratch.as<float>(), 1, d.stream), what, need > 0 ? 2 : 1);
+    check(jb_gemm_simt(a, a_dt, w, w_dt, out, n, m, k, scratch.as<float>(), 1, d.stream), what, need > 0 ? 2 : 1);
 }
 
 Stack linear(Device &d, const void *a, DType a_dt, long long n, long long k, const DevTensor &w,

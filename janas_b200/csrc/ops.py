@@ -1210,10 +1210,10 @@ def linear(a: torch.Tensor, weight: torch.Tensor, force_simt: bool = False,
     out = torch.empty((1, n, m), dtype=torch.float32, device=a.device)
     if (not force_simt and a.dtype == torch.float32 and weight.dtype == torch.float32
             and L.jb_gemm_f32_tc_ok(_p(weight), m, k)):
-        need = int(L.jb_gemm_f32_tc_scratch(n, m, k))
-        scratch = torch.empty((need,), dtype=torch.float32, device=a.device) if need else None
-        _check(L.jb_gemm_f32_tc(_p(a), _p(weight), _p(out), n, m, k, _p(scratch), 0, _stream()),
-               "linear (float, tcgen05)", kernels=int(L.jb_gemm_f32_tc_launches(n, m, k)))
+        have = int(L.jb_gemm_f32_tc_scratch(n, m, k))
+        scratch = torch.empty((have,), dtype=torch.float32, device=a.device) if have else None
+        _check(L.jb_gemm_f32_tc(_p(a), _p(weight), _p(out), n, m, k, _p(scratch), have, 0, _stream()),
+               "linear (float, tcgen05)", kernels=int(L.jb_gemm_f32_tc_launches(n, m, k, have)))
         return out
     need = int(L.jb_gemm_simt_scratch(n, m, k))
     scratch = torch.empty((need,), dtype=torch.float32, device=a.device) if need else None

@@ -97,7 +97,7 @@ static size_t size_class(size_t b) {
     return (b + step - 1) / step * step;
 }
 
-Buf Pool::get(size_t bytes) {
+Buf Pool::take(size_t bytes, bool must) {
     size_t cap = size_class(bytes);
     auto it = free_.find(cap);
     if (it != free_.end() && !it->second.empty()) {
@@ -107,6 +107,10 @@ Buf Pool::get(size_t bytes) {
     }
     void *p = nullptr;
     cudaError_t e = cudaMalloc(&p, cap);
+    if (e == cudaErrorMemoryAllocation && !must) {
+        cudaGetLastError();
+        return Buf();
+    }
     if (e == cudaErrorMemoryAllocation) {
         // what lies idle in other size classes may make room (the stream is drained
         // first: idle buffers may still be read by kernels that are under way)
@@ -120,6 +124,10 @@ Buf Pool::get(size_t bytes) {
     allocations_++;
     return Buf(p, bytes, cap, this);
 }
+
+Buf Pool::get(size_t bytes) { return take(bytes, true); }
+
+Buf Pool::get_if_room(size_t bytes) { return take(bytes, false); }
 
 void Pool::put(void *p, size_t cap) { free_[cap].push_back(p); }
 

@@ -74,6 +74,7 @@ class Pool {
 public:
     ~Pool();
     Buf get(size_t bytes);
+    Buf get_if_room(size_t bytes);  // empty where the device has no memory left for it; frees nothing for it
     void put(void *p, size_t cap);
     void trim();                    // frees what is idle; the caller has synchronized
     // called at the start of trim(): whoever holds addresses of pool buffers beyond a
@@ -83,6 +84,7 @@ public:
     long long allocations() const { return allocations_; }   // cudaMalloc calls so far
 
 private:
+    Buf take(size_t bytes, bool must);
     std::map<size_t, std::vector<void *>> free_;
     size_t reserved_ = 0;
     long long allocations_ = 0;
@@ -124,6 +126,7 @@ public:
     cudaStream_t stream = nullptr;
     Pool pool;
     long long h2d_bytes = 0;        // bytes of step inputs copied to the device so far
+    size_t parts_scratch_limit = ~(size_t)0;   // lowered when the device had no room for a float product's scratch
 
 private:
     struct Stage { void *host = nullptr; size_t cap = 0; cudaEvent_t done = nullptr; bool used = false; };

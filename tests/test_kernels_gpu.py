@@ -198,6 +198,22 @@ def test_gemm_f32_parts(m, k):
     assert ops().gemm_tc_error() == 0
 
 
+@pytest.mark.parametrize("m,k,n", [(2560, 4096, 321), (640, 9728, 100), (19000, 1100, 33), (600, 1028, 16)])
+def test_gemm_f32_parts_with_less_scratch(m, k, n):
+    """Less scratch than a call asks for, and none: more passes over the rows, tiles not shared out, the same bits."""
+    L = ops().lib()
+    a, w = rnd(n, k).to(DEV), rnd(m, k, seed=3).to(DEV)
+    want = ops().linear(a, w)[0]
+    full = int(L.jb_gemm_f32_tc_scratch(n, m, k))
+    for have in (full, full - 1, full // 2, full // 7, 0):
+        scratch = torch.full((max(have, 4),), math.nan, device=DEV)
+        got = torch.full((n, m), math.nan, device=DEV)
+        assert L.jb_gemm_f32_tc(a.data_ptr(), w.data_ptr(), got.data_ptr(), n, m, k, scratch.data_ptr() if have else None,
+                                have, 0, torch.cuda.current_stream().cuda_stream) == 0
+        assert torch.equal(got, want), have
+    assert ops().gemm_tc_error() == 0
+
+
 @pytest.mark.parametrize("n", [7, 40])
 @pytest.mark.parametrize("up_a,up_w", [(-100, 0), (-113, 0), (-120, 0), (-126, 0), (0, -113), (0, -126), (-63, -63), (40, 30)])
 def test_gemm_f32_parts_of_small_floats(n, up_a, up_w):

@@ -69,3 +69,14 @@ def test_which_float_products_go_in_parts():
     assert ok(0, 512, 1024) and ok(0, 513, 1028) and ok(0, 151936, 2560) and ok(0, 512, 1 << 17)
     assert not ok(0, 511, 1024) and not ok(0, 512, 1020) and not ok(0, 512, 1026) and not ok(4, 512, 1024)
     assert not ok(0, 512, (1 << 17) + 4)
+
+
+@pytest.mark.parametrize("m,k", [(6144, 2560), (2560, 9728), (151936, 2560), (512, 32768), (18944, 65536), (513, 1028)])
+def test_scratch_of_float_products_is_bounded(m, k):
+    """At most 72 MiB whatever the rows (host code; asked without a GPU too), and a plan for less, down to none."""
+    L = ops.lib()
+    for n in (1, 16, 17, 33, 60, 161, 300, 1000, 2048, 5001, 40000):
+        need = L.jb_gemm_f32_tc_scratch(n, m, k)
+        assert 0 <= need * 4 <= 72 << 20, (n, need)
+        few, many = L.jb_gemm_f32_tc_launches(n, m, k, need), L.jb_gemm_f32_tc_launches(n, m, k, 0)
+        assert 1 <= few and many == -(-n // 32), (n, few, many)
