@@ -47,8 +47,8 @@ namespace ops {
 // how many of the library's kernels have been launched (for measurements)
 long long launches();
 void count_launches(long long n);
-// n 32-bit words between pinned host memory and the device, in the stream's order.  src_early: nothing that may still
-// be running writes src.
+// n 32-bit words between pinned host memory and the device, in the stream's order: up to 1 MB by a kernel, larger arrays
+// at a copy engine's pace.  src_early: nothing that may still be running writes src.
 void copy_words(Device &d, const void *src, void *dst, long long n, bool src_early);
 
 int attention_chunk();

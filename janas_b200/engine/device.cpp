@@ -212,8 +212,7 @@ void Device::upload_pinned(void *dst, const void *src, size_t bytes) {
     Stage *s = nullptr;
     if (last_ >= 0 && ring_[(size_t)last_].host == src) s = &ring_[(size_t)last_];
     if (!s) fail(JB_LLM_EFAIL, "upload_pinned: not the buffer that pinned() gave last");
-    // small arrays of whole words by a kernel (see jb_copy_words); what is large goes at the copy engine's pace
-    if (bytes % 4 == 0 && bytes <= (256u << 10) && (uintptr_t)dst % 4 == 0 && bytes > 0)
+    if (bytes % 4 == 0 && (uintptr_t)dst % 4 == 0 && bytes > 0)
         ops::copy_words(*this, src, dst, (long long)(bytes / 4), true);
     else if (bytes)
         cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream), "copy to the device");

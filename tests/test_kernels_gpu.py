@@ -267,6 +267,23 @@ def test_gemm_f32_parts_nothing_finite(m, k, n, what):
     assert ops().gemm_tc_error() == 0
 
 
+@pytest.mark.parametrize("words", [1, 255, 256, 257, 5000, 262144])
+def test_copy_words(words):
+    """Between pinned host memory and the device, both ways, right behind a kernel that writes the source; only the
+    words that are asked for; no odd addresses."""
+    L = ops().lib()
+    st = torch.cuda.current_stream().cuda_stream
+    host = torch.randint(-2 ** 31, 2 ** 31 - 1, (words,), dtype=torch.int32).pin_memory()
+    back = torch.zeros(words + 3, dtype=torch.int32).pin_memory()
+    dev = torch.full((words + 3,), 77, dtype=torch.int32, device=DEV)
+    assert L.jb_copy_words(host.data_ptr(), dev[1:].data_ptr(), words, 1, st) == 0
+    assert L.jb_copy_words(dev.data_ptr(), back.data_ptr(), words + 3, 0, st) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(back[1:words + 1], host) and back[0] == 77 and (back[words + 1:] == 77).all()
+    assert L.jb_copy_words(host.data_ptr(), dev.data_ptr() + 2, 1, 1, st) != 0
+    assert L.jb_copy_words(host.data_ptr(), dev.data_ptr(), 0, 1, st) == 0
+
+
 @pytest.mark.parametrize("odt", DTYPES)
 def test_swiglu(odt):
     n, ff = 7, 300
