@@ -1077,15 +1077,8 @@ attn_tc_decode_kernel(const __grid_constant__ CUtensorMap map_q,
                 hi.x = (hi.x * sc) * wh.x; hi.y = (hi.y * sc) * wh.y;
                 hi.z = (hi.z * sc) * wh.z; hi.w = (hi.w * sc) * wh.w;
             }
-            if (!is_v && f.cs != nullptr) {
-                // (spelled out as the compiler takes the rope kernel's: left to it, either product may be the one
-                // that is rounded)
-                float4 a = lo, b = hi;
-                lo = make_float4(fmaf(a.x, co.x, -__fmul_rn(b.x, si.x)), fmaf(a.y, co.y, -__fmul_rn(b.y, si.y)),
-                                 fmaf(a.z, co.z, -__fmul_rn(b.z, si.z)), fmaf(a.w, co.w, -__fmul_rn(b.w, si.w)));
-                hi = make_float4(fmaf(a.x, si.x, __fmul_rn(b.x, co.x)), fmaf(a.y, si.y, __fmul_rn(b.y, co.y)),
-                                 fmaf(a.z, si.z, __fmul_rn(b.z, co.z)), fmaf(a.w, si.w, __fmul_rn(b.w, co.w)));
-            }
+            if (!is_v && f.cs != nullptr)
+                turn4(lo, hi, co, si);
             if (is_q) {
                 // where the TMA load would have put it: block of the half, row of the
                 // head, 16-byte chunk at4 / 8 of the row in the 128-byte swizzle

@@ -150,6 +150,21 @@ __device__ __forceinline__ void split2(f32x2 v, float &lo, float &hi)
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
+// x c + y s, the second product rounded by itself: half of a rotation.  Every kernel that rotates the q and k of a
+// fused product calls it, so that prompts, steps of few rows and the decode attention, which makes its own, give the
+// same bits whichever product a compiler would have rounded.
+__device__ __forceinline__ float turned(float x, float c, float y, float s) { return fmaf(x, c, __fmul_rn(y, s)); }
+
+// (lo, hi) -> (lo c - hi s, lo s + hi c), four pairs.
+__device__ __forceinline__ void turn4(float4 &lo, float4 &hi, const float4 &c, const float4 &s)
+{
+    const float4 a = lo, b = hi;
+    lo = make_float4(turned(a.x, c.x, -b.x, s.x), turned(a.y, c.y, -b.y, s.y), turned(a.z, c.z, -b.z, s.z),
+                     turned(a.w, c.w, -b.w, s.w));
+    hi = make_float4(turned(a.x, s.x, b.x, c.x), turned(a.y, s.y, b.y, c.y), turned(a.z, s.z, b.z, c.z),
+                     turned(a.w, s.w, b.w, c.w));
+}
+
 // Programmatic dependent launch.  Every kernel of this library is launched with
 // the attribute that lets its CTAs start while the kernel before it in the
 // stream is still running.  pdl_trigger() (early in a kernel) allows the next

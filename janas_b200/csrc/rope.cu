@@ -130,8 +130,8 @@ qk_norm_rope_append_kernel(
                 b = (b * scale) * wh[j];
             }
             if (rotate) {
-                dst[i] = from_f<TC>(a * co[j] - b * si[j]);
-                dst[i + half] = from_f<TC>(a * si[j] + b * co[j]);
+                dst[i] = from_f<TC>(turned(a, co[j], -b, si[j]));
+                dst[i + half] = from_f<TC>(turned(a, si[j], b, co[j]));
             } else {
                 dst[i] = from_f<TC>(a);
                 dst[i + half] = from_f<TC>(b);
@@ -243,13 +243,8 @@ qk_norm_rope_append_vec_kernel(
             hi.x = (hi.x * scale) * wh.x; hi.y = (hi.y * scale) * wh.y;
             hi.z = (hi.z * scale) * wh.z; hi.w = (hi.w * scale) * wh.w;
         }
-        if (rotate) {
-            float4 a = lo, b = hi;
-            lo = make_float4(a.x * co.x - b.x * si.x, a.y * co.y - b.y * si.y,
-                             a.z * co.z - b.z * si.z, a.w * co.w - b.w * si.w);
-            hi = make_float4(a.x * si.x + b.x * co.x, a.y * si.y + b.y * co.y,
-                             a.z * si.z + b.z * co.z, a.w * si.w + b.w * co.w);
-        }
+        if (rotate)
+            turn4(lo, hi, co, si);
         store4(dst + at4, lo);
         store4(dst + half + at4, hi);
     }
@@ -353,13 +348,8 @@ qk_norm_rope_append_row_kernel(
                 h.x = (h.x * scale) * wh.x; h.y = (h.y * scale) * wh.y;
                 h.z = (h.z * scale) * wh.z; h.w = (h.w * scale) * wh.w;
             }
-            if (!is_v && has_rot) {
-                float4 a = l, b = h;
-                l = make_float4(a.x * co.x - b.x * si.x, a.y * co.y - b.y * si.y,
-                                a.z * co.z - b.z * si.z, a.w * co.w - b.w * si.w);
-                h = make_float4(a.x * si.x + b.x * co.x, a.y * si.y + b.y * co.y,
-                                a.z * si.z + b.z * co.z, a.w * si.w + b.w * co.w);
-            }
+            if (!is_v && has_rot)
+                turn4(l, h, co, si);
             store4(dst, l);
             store4(dst + half, h);
         }
@@ -449,7 +439,7 @@ qkv_prepare_append_kernel(const float *__restrict__ qkv, int S, size_t split_str
                 int f = pairs ? i >> 1 : low ? i : j;
                 float co = cs[(size_t)pos * rot_half + f], si = sn[(size_t)pos * rot_half + f];
                 // (a, b) -> (a cos - b sin, b cos + a sin), a the lower value of the pair
-                v = low ? v * co - u * si : v * co + u * si;
+                v = turned(v, co, low ? -u : u, si);
             }
             if (pass == 0)
                 ss2 = fmaf(v, v, ss2);
@@ -546,8 +536,8 @@ qkv_prepare_append_vec_kernel(const float *__restrict__ qkv, int S, size_t split
     }
     if (pairs) {
         if (!is_v && 2 * l < rot_half)
-            v = make_float4(v.x * co.x - v.y * si.x, v.y * co.x + v.x * si.x, v.z * co.y - v.w * si.y,
-                            v.w * co.y + v.z * si.y);
+            v = make_float4(turned(v.x, co.x, -v.y, si.x), turned(v.y, co.x, v.x, si.x), turned(v.z, co.y, -v.w, si.y),
+                            turned(v.w, co.y, v.z, si.y));
     } else if (rot_half > 0) {
         int pl = group0 + (l < hl ? l + hl : l < 2 * hl ? l - hl : l);
         float4 u;
@@ -557,11 +547,11 @@ qkv_prepare_append_vec_kernel(const float *__restrict__ qkv, int S, size_t split
         u.w = __shfl_sync(0xffffffffu, v.w, pl);
         // (a, b) -> (a cos - b sin, b cos + a sin), a the lower value of the pair
         if (l < hl)
-            v = make_float4(v.x * co.x - u.x * si.x, v.y * co.y - u.y * si.y, v.z * co.z - u.z * si.z,
-                            v.w * co.w - u.w * si.w);
+            v = make_float4(turned(v.x, co.x, -u.x, si.x), turned(v.y, co.y, -u.y, si.y), turned(v.z, co.z, -u.z, si.z),
+                            turned(v.w, co.w, -u.w, si.w));
         else if (l < 2 * hl)
-            v = make_float4(v.x * co.x + u.x * si.x, v.y * co.y + u.y * si.y, v.z * co.z + u.z * si.z,
-                            v.w * co.w + u.w * si.w);
+            v = make_float4(turned(v.x, co.x, u.x, si.x), turned(v.y, co.y, u.y, si.y), turned(v.z, co.z, u.z, si.z),
+                            turned(v.w, co.w, u.w, si.w));
     }
     if (unit) {
         // a norm without a weight after the rotation, on q and k heads

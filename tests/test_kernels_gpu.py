@@ -481,6 +481,30 @@ def test_attention_many_kept_tokens_before_the_window_moves(dtype, keep_first):
     assert torch.equal(run(window, keep_first), run(0, 0))
 
 
+@pytest.mark.parametrize("n,hd", [(9, 48), (9, 128), (300, 128), (12, 64)])
+def test_rotation_rounds_the_same_product_everywhere(n, hd):
+    """lo c - hi s and lo s + hi c with the second product rounded by itself and the first not, in every kernel that
+    rotates: factors of twelve bits, so that what is left is exact in 64 bits and the other choice shows."""
+    nh, nkv, half = 4, 1, hd // 2
+    short = lambda t: (t.view(torch.int32) & ~0xfff).view(torch.float32)
+    qkv = rnd(1, n, (nh + 2 * nkv) * hd)
+    qkv.view(n, nh + 2 * nkv, 2, half)[:, :, 0] = short(qkv.view(n, nh + 2 * nkv, 2, half)[:, :, 0].contiguous())
+    cs, sn = short(rnd(512, half, seed=5)), short(rnd(512, half, seed=6))
+    pos, seq = torch.arange(n, dtype=torch.int32), torch.zeros(n, dtype=torch.int32)
+    bt = torch.arange(8, dtype=torch.int32)[None]
+    kc = torch.zeros(8, nkv, 64, hd, device=DEV)
+    q = ops().qk_norm_rope_append(qkv.to(DEV), None, None, 1e-6, cs.to(DEV), sn.to(DEV), pos.to(DEV), seq.to(DEV),
+                                  bt.to(DEV), kc, torch.zeros_like(kc), nh, nkv, hd, torch.float32).cpu()
+    x = qkv.view(n, nh + 2 * nkv, 2, half)[:, :nh + nkv]
+    lo, hi, c, s = x[:, :, 0], x[:, :, 1], cs[:n, None], sn[:n, None]
+    want = torch.cat([(lo.double() * c - (hi * s).double()).float(), (lo.double() * s + (hi * c).double()).float()], -1)
+    other = (lo.double() * c - hi.double() * s).float()
+    assert (want[..., :half] != other).sum() > 100
+    assert torch.equal(q.view(n, nh, hd), want[:, :nh])
+    keys = kc.cpu()[:, 0].reshape(-1, hd)[:n]
+    assert torch.equal(keys, want[:, nh])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n0,n1,hd,nh,nkv", [(25, 15, 48, 6, 2), (300, 58, 128, 6, 2), (3, 1, 16, 6, 2),
                                              (40, 9, 32, 5, 1), (17, 30, 64, 9, 3),
