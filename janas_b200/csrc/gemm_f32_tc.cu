@@ -43,6 +43,7 @@ constexpr int F_BK = 64;                       // k of a block
 constexpr int F_M = 128;                       // features of a tile
 constexpr int BOX_K = 32;                      // k of a box of weights: 128 bytes of float, one swizzle row
 constexpr int BOX_BYTES = F_M * BOX_K * 4;
+static_assert(BOX_K * 4 == 128 && F_BK * 2 == 128, "boxes of tensor_map_2d");
 constexpr int A_COLS = 3 * F_BK / 2;           // tensor-memory columns of a block's weights: three parts, two values a column
 
 __device__ int g_gemm_f32_tc_error;            // 0, or the code of the first wait that ran out
@@ -870,12 +871,12 @@ static int f32_run(const F32Plan &p, const float *A, const float *W, float *out,
     work.units = (int)(p.whole + p.rest * p.segments);
     const int a_vec = (uintptr_t)A % 16 == 0, kp = (k + 7) / 8 * 8;
     CUtensorMap map_w, map_a;
-    if (!tensor_map_2d(W, m, k, F_M, BOX_K, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, &map_w))
+    if (!tensor_map_2d(W, m, k, F_M, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, &map_w))
         return JB_EINVAL;
     map_a = map_w;
     float *part = p.part_floats > 0 ? scratch + p.plane_floats : nullptr;
     if (p.plane_floats > 0) {
-        if (!tensor_map_2d(scratch, 3 * n, kp, p.bn, F_BK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, &map_a))
+        if (!tensor_map_2d(scratch, 3 * n, kp, p.bn, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, &map_a))
             return JB_EINVAL;
         launch(f32_parts_kernel, (unsigned)(((size_t)n * (kp / 4) + 255) / 256), 256, 0, st, A, (bf16 *)scratch, n, k, kp,
                a_vec);

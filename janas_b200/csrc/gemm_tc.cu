@@ -441,8 +441,7 @@ EncodeTiled tensor_map_encoder()
     return fn;
 }
 
-bool tensor_map_2d(const void *ptr, int rows, int k, int box_rows, int box_k, CUtensorMapDataType type,
-                   CUtensorMap *out)
+bool tensor_map_2d(const void *ptr, int rows, int k, int box_rows, CUtensorMapDataType type, CUtensorMap *out)
 {
     typedef std::tuple<const void *, int, int, int, int> Key;
     static std::map<Key, CUtensorMap> cache;
@@ -458,8 +457,9 @@ bool tensor_map_2d(const void *ptr, int rows, int k, int box_rows, int box_k, CU
     if (!enc)
         return false;
     cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)k * (type == CU_TENSOR_MAP_DATA_TYPE_FLOAT32 ? 4 : 2)};
-    cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
+    const int bytes = type == CU_TENSOR_MAP_DATA_TYPE_FLOAT32 ? 4 : 2;
+    cuuint64_t strides[1] = {(cuuint64_t)k * bytes};
+    cuuint32_t box[2] = {(cuuint32_t)(128 / bytes), (cuuint32_t)box_rows};      // one row of the swizzle
     cuuint32_t estr[2] = {1, 1};
     CUtensorMap map;
     if (enc(&map, type, 2, const_cast<void *>(ptr), dims, strides, box,
@@ -473,9 +473,10 @@ bool tensor_map_2d(const void *ptr, int rows, int k, int box_rows, int box_k, CU
     return true;
 }
 
+static_assert(BK * 2 == 128, "boxes of tensor_map_2d");
 static bool tensor_map(const void *ptr, int rows, int k, int box_rows, CUtensorMap *out)
 {
-    return tensor_map_2d(ptr, rows, k, box_rows, BK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out);
+    return tensor_map_2d(ptr, rows, k, box_rows, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out);
 }
 
 template <int BN, int MT, int EPI>

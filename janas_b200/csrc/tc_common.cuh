@@ -316,9 +316,8 @@ typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, 
                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiled tensor_map_encoder();
-// A [rows, k] row-major matrix of bfloat16 or float, read in boxes of box_rows x box_k (128 bytes) with the
+// A [rows, k] row-major matrix of bfloat16 or float, read in boxes of box_rows x 128 bytes (64 or 32 of k) with the
 // 128-byte swizzle; what lies outside the matrix reads as zero.
-bool tensor_map_2d(const void *ptr, int rows, int k, int box_rows, int box_k, CUtensorMapDataType type,
-                   CUtensorMap *out);
+bool tensor_map_2d(const void *ptr, int rows, int k, int box_rows, CUtensorMapDataType type, CUtensorMap *out);
 
 }  // namespace jb

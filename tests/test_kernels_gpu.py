@@ -198,6 +198,52 @@ def test_gemm_f32_parts(m, k):
     assert ops().gemm_tc_error() == 0
 
 
+@pytest.mark.parametrize("m,k", [(600, 1100), (2560, 2560), (640, 9728)])
+@pytest.mark.parametrize("n", [8, 100])
+def test_gemm_f32_parts_as_a_whole(m, k, n):
+    """The error of the whole product against 64 bits (measured: 1.0e-7 to 1.3e-7 of it; 4.4e-6 with two parts a float
+    and three products): at most 3e-7, and no more than the plain kernel's."""
+    a, w = rnd(n, k).to(DEV), rnd(m, k, seed=3).to(DEV)
+    want = a.double() @ w.double().T
+    off = lambda got: float((got.double() - want).norm() / want.norm())
+    got = off(ops().linear(a, w)[0])
+    assert got <= 3e-7 and got <= off(ops().linear(a, w, force_simt=True)[0])
+
+
+def each_product_alone(n, m, k):
+    """Operands whose sums are one product of parts each: a row of the tokens holds x1, x1, x2, x2 at four places, one
+    of the weights y1, -y2, -y1, y2, and the sum is (x1 - x2)(y1 - y2), where a difference is all that one part adds.
+    Places in every quarter of a block, rows times powers of two, exact in every step.  Returns tokens, weights and the
+    wanted sums; of the pairs whose product is left out (mid lo, lo mid, lo lo) NaN."""
+    mid, lo = 2.0 ** -9, 2.0 ** -18
+    pairs = [(1.0, 0.0), (1 + mid, 1.0), (1 + mid + lo, 1 + mid)]
+    a, w, want = torch.zeros(n, k), torch.zeros(m, k), torch.zeros(n, m, dtype=torch.float64)
+    places = [0, 20, 44, 60, 64 * (k // 64 // 2) + 32, k - 4]
+    for r in range(n):
+        x1, x2 = pairs[r % 3]
+        for i in places[r % 2::2]:
+            a[r, i:i + 4] = torch.tensor([x1, x1, x2, x2]) * 2.0 ** [0, 50, -60, -100, -126][r // 3 % 5]
+    for f in range(m):
+        y1, y2 = pairs[f % 3]
+        i = places[f // 3 % len(places)]
+        w[f, i:i + 4] = torch.tensor([y1, -y2, -y1, y2]) * (-1.0 if f // 7 % 2 else 1.0)
+    for pa in range(3):
+        for pw in range(3):
+            rows, feats = torch.arange(pa, n, 3), torch.arange(pw, m, 3)
+            want[rows[:, None], feats] = a[rows].double() @ w[feats].double().T if pa + pw <= 2 else math.nan
+    return a, w, want
+
+
+@pytest.mark.parametrize("n", [15, 60])
+def test_gemm_f32_parts_every_product(n):
+    """Each of the six products of parts by itself, exact: one that is left out or taken twice shows."""
+    a, w, want = each_product_alone(n, 600, 1100)
+    got = ops().linear(a.to(DEV), w.to(DEV))[0].cpu().double()
+    told = ~want.isnan()
+    assert torch.equal(got[told], want[told])
+    assert (want[told] != 0).sum() > 100
+
+
 @pytest.mark.parametrize("m,k,n", [(2560, 4096, 321), (640, 9728, 100), (19000, 1100, 33), (600, 1028, 16)])
 def test_gemm_f32_parts_with_less_scratch(m, k, n):
     """Less scratch than a call asks for, and none: more passes over the rows, tiles not shared out, the same bits."""
