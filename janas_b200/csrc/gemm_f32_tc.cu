@@ -19,13 +19,15 @@
 // operand, in shared memory.  For few tokens some warps of the CTA make them from the floats; for many a kernel
 // ahead of this one does it once, instead of every tile of features again, and TMA brings them.
 //
-// What bounds it: few tokens, the weights' bytes (19456 x 2560 at 8 tokens 4.5 TB/s; a block's 24 MMAs take about 1,000
-// cycles beside the stores of the next block's parts, its 32 KB of weights 1,400 at the memory's full rate); many, the
-// MMAs: 1,920 cycles a block of 160 tokens, of 2,150 that it takes.  One B200, microseconds, weights from memory, all
-// kernels of a call; in brackets gemm_simt.cu, which took these products before:
-//   tokens 8:    6144 x 2560  16.9 (20.6)  2560 x 4096  14.4 (14.6)  19456 x 2560  44.1 (50.7)  2560 x 9728  23.2 (28.5)
-//   tokens 64:   6144 x 2560  22.0 (65.4)  2560 x 4096  18.7 (45.6)  19456 x 2560  58.1 (207)   2560 x 9728  30.0 (117)
-//   tokens 300:  6144 x 2560  57.0 (271)   2560 x 4096  45.6 (172)   19456 x 2560  171 (724)    2560 x 9728  83.4 (414)
+// What bounds it: few tokens, the stores of the next block's parts into tensor memory beside a block's MMAs (24 MMAs of 16
+// tokens take 590 cycles alone, about 1,000 beside the stores; a block some 1,600 with all of it, its 32 KB of weights
+// 1,400 at the memory's full rate); many, the MMAs: 1,920 cycles a block of 160 tokens, of 2,150 that it takes.  One
+// B200, microseconds, weights from memory, all kernels of a call; in brackets gemm_simt.cu, which took these products
+// before:
+//   tokens          6144 x 2560   2560 x 4096   19456 x 2560   2560 x 9728   151936 x 2560
+//       8           17.5 (21.2)   14.8 (15.1)   47.6 (52.6)    24.2 (29.5)   306 to 324 (272)
+//      64           22.6 (67.4)   19.1 (45.9)   59.6 (208)     31.0 (118)    380 (1,150)
+//     300           56.2 (271)    44.7 (171)    170 (724)      82.3 (414)    1,270 (5,290)
 // The error against 64 bits is 1.0e-7 to 1.3e-7 of the result (2.9e-7 to 3.0e-7), also where all of a token or of a
 // feature is small.
 //
@@ -821,8 +823,15 @@ static int f32_launch(const CUtensorMap &map_w, const CUtensorMap &map_a, const 
 
 using namespace jb;
 
-// Whether this kernel takes a product; says nothing about n, so that a row's bits do not depend on the batch.  Smaller
-// weights are left to the plain kernel: at 8 tokens 512 x 1024 takes 7.3 us (7.8 there) and 1000 x 1028 7.5 (7.8), but
+// Whether this kernel takes a product; says nothing about n, so that a row's bits do not depend on the batch.  That costs
+// a step of 1 to 8 rows a little where the weight has few tiles and moderate k, or is a head: in a captured chain of norm
+// and product, us, this kernel and gemm_simt.cu, 1 / 8 / 16 / 32 rows: 2560 x 4096 15.7 / 16.8 / 17.2 / 19.3 and
+// 14.9 / 15.4 / 20.9 / 35.2; 2048 x 6144 16.5 / 18.0 / 18.6 / 20.2 and 15.7 / 16.1 / 21.6 / 35.7; 4096 x 2560 14.2 /
+// 15.0 / 15.6 / 17.0 and 14.1 / 14.6 / 20.1 / 34.3; a head of 151,936 x 2560 269 to 290 / 264 to 284 / 293 / 318 to 345
+// and 266 / 270 / 367 / 620 (by box: it is the clock's, the plain kernel's is the memory's).  Everything else measured is
+// ahead from one row on (19456 x 2560 46 / 47 / 48 / 55 and 50 / 53 / 72 / 110), all of them are from 16 rows on, and a
+// prompt takes a quarter of the time.  A whole 36-layer step of 8 rows: 5.73 ms, 5.83 by plain multiply-adds.
+// Smaller weights are left to the plain kernel: at 8 tokens 512 x 1024 takes 7.3 us (7.8 there) and 1000 x 1028 7.5 (7.8), but
 // 512 x 512 7.2 (6.7), 2560 x 512 7.4 (6.8) and 256 x 256 5.4 (3.9).  Longer rows too: a tile whose sums are all infinite
 // takes the epilogue some 4,500 cycles a k (23 ms at 9,728), and the others' waits end after 2 * 10^9.
 extern "C" int jb_gemm_f32_tc_ok(const void *W, int m, int k)

@@ -108,9 +108,9 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // Four MMAs along k, the operands' descriptors SA and SB (units of 16 bytes) apart; accumulate: whether the first one
-// adds to d.  By a whole warp whose lanes agree on the arguments: one of them is elected to issue.  (In a branch that a
-// single lane takes, or with an election each, every instruction waits for its operands to be moved into uniform
-// registers: 40 to 64 cycles an MMA, measured, where one of 16 tokens runs for about 25 and one of 128 for 64.)
+// adds to d.  By a whole warp whose lanes agree on the arguments: one of them is elected to issue.  (Issued in a branch
+// that a single lane takes, or with an election each, an MMA takes 40 to 64 cycles, measured; like this one of 16 tokens
+// about 25 and one of 128 64.)
 template <int SA, int SB>
 __device__ __forceinline__ void tc_mma4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate)
