@@ -51,6 +51,7 @@ Engine::~Engine() {
         dev->pool.before_trim = nullptr;
     }
     graphs_.clear();
+    retired_.clear();
 }
 
 static std::unique_ptr<Engine> make_engine(std::unique_ptr<ArchConfig> cfg, DType dtype, long long max_tokens,
@@ -264,9 +265,24 @@ Buf Engine::step(const std::vector<StepEntry> &entries, long long *n_wanted) {
 void Engine::drop_graphs() {
     if (graphs_.empty()) return;
     cudaStreamSynchronize(dev->stream);
-    graphs_.clear();
+    for (auto it = graphs_.begin(); it != graphs_.end();) {
+        if (it->second.get() == starting_) {
+            it->second->let_go();
+            ++it;
+        } else {
+            retire(std::move(it->second));
+            it = graphs_.erase(it);
+        }
+    }
     last_graph_ = nullptr;
     last_slots_.clear();
+}
+
+void Engine::retire(std::unique_ptr<DecodeGraph> g) {
+    g->let_go();
+    if (g->unread()) retired_.push_back(std::move(g));
+    retired_.remove_if([](const std::unique_ptr<DecodeGraph> &r) { return !r->unread(); });
+    while (retired_.size() > 64) retired_.pop_front();      // handles that nobody came back for
 }
 
 SamplerScratch &Engine::sampler_scratch() {
@@ -387,6 +403,7 @@ PendingDecode *Engine::decode_begin(const std::vector<int> &slots, const int32_t
                 last_slots_.clear();
                 if (!tokens) fail(JB_LLM_EFAIL, "the step before this one lost its graph");
             }
+            retire(std::move(graphs_.front().second));
             graphs_.pop_front();
         }
         graphs_.emplace_back(key, std::unique_ptr<DecodeGraph>(
@@ -394,6 +411,12 @@ PendingDecode *Engine::decode_begin(const std::vector<int> &slots, const int32_t
         g = graphs_.back().second.get();
     }
     DecodeGraph *before = tokens ? nullptr : last_graph_;
+    // (a pool that runs out of memory lets go of captured steps, and this one may be asking)
+    struct Starting {
+        DecodeGraph *&at;
+        Starting(DecodeGraph *&a, DecodeGraph *graph) : at(a) { at = graph; }
+        ~Starting() { at = nullptr; }
+    } starting(starting_, g);
     PendingDecode *pending = g->begin(slots, tokens ? p.tokens.data() : nullptr, p.pos0, before);
     last_graph_ = g;
     last_slots_ = slots;

@@ -156,6 +156,10 @@ private:
     // used last at the back, the oldest goes when there are more than max_graphs
     using GraphKey = std::tuple<int, long long, bool, bool>;
     std::list<std::pair<GraphKey, std::unique_ptr<DecodeGraph>>> graphs_;
+    void retire(std::unique_ptr<DecodeGraph> g);
+    // graphs that were let go of while a caller still had the tokens of a step to take
+    std::list<std::unique_ptr<DecodeGraph>> retired_;
+    DecodeGraph *starting_ = nullptr;       // the graph whose step is being launched: stays, whoever drops graphs
     DecodeGraph *last_graph_ = nullptr;     // the graph of the decode step begun last
     std::vector<int> last_slots_;
     std::vector<int> cache_entry_;          // run-order entry -> entry whose cache it uses, or -1

@@ -18,9 +18,19 @@ DecodeGraph::DecodeGraph(Engine &e, int batch, long long bound, bool sampled, bo
     dev_ = e.dev->tensor(I32, {(long long)total_}, true);
 }
 
-DecodeGraph::~DecodeGraph() {
+void DecodeGraph::let_go() {
     if (exec_) cudaGraphExecDestroy(exec_);
     if (graph_) cudaGraphDestroy(graph_);
+    exec_ = nullptr;
+    graph_ = nullptr;
+}
+
+bool DecodeGraph::unread() const {
+    return (used_[0] && !pending_[0].taken) || (used_[1] && !pending_[1].taken);
+}
+
+DecodeGraph::~DecodeGraph() {
+    let_go();
     for (int i = 0; i < 2; i++) {
         if (events_[i]) cudaEventDestroy(events_[i]);
         if (host_[i]) cudaFreeHost(host_[i]);

@@ -34,6 +34,11 @@ public:
     PendingDecode *begin(const std::vector<int> &slots, const int32_t *tokens,
                          const std::vector<long long> &pos0, DecodeGraph *before);
 
+    // Forgets the captured step (the next one captures again); the device is idle.
+    void let_go();
+    // Whether a step's tokens have not been taken yet: its PendingDecode is this object's.
+    bool unread() const;
+
     int kernels = 0;        // kernels per replay
 
 private:

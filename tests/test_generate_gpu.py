@@ -187,6 +187,36 @@ def test_replayed_decode_steps_equal_launched_ones(dtype):
         m.engine.cache.check()
 
 
+def test_tokens_of_a_step_outlive_its_captured_form():
+    """A decode step under way, its graph dropped, trimmed away or pushed out by another shape before its tokens are
+    taken: the tokens are there all the same."""
+    from janas_b200.engine import Engine, StepEntry
+    rng = np.random.default_rng(6)
+    prompts = [tokens(rng, n, TINY["E"]["vocab_size"]) for n in (250, 40)]
+
+    def run(between):
+        eng = Engine.open(model_dir("E"), dtype="bfloat16", max_tokens=1024, max_seqs=2, n_ctx=512)
+        eng.set_max_graphs(1)
+        slots = [eng.new_sequence() for _ in prompts]
+        eng.step_numpy([StepEntry(s, p) for s, p in zip(slots, prompts)])
+        out, ahead = [], None
+        for i in range(12):                 # the first sequence passes position 256: another graph
+            step = eng.decode_begin(slots, [3 + i, 5 + i])
+            if between:
+                between(eng, i)
+            if ahead is not None:
+                out.append(ahead.result())
+            ahead = step
+        out.append(ahead.result())
+        eng.check()
+        eng.close()
+        return np.stack(out)
+
+    want = run(None)
+    assert np.array_equal(run(lambda e, i: e.drop_graphs() if i % 3 == 1 else None), want)
+    assert np.array_equal(run(lambda e, i: e._set(trim=True) if i % 4 == 2 else None), want)
+
+
 def test_old_decode_graphs_are_dropped_and_captured_again():
     """No more than ``max_graphs`` captured steps are kept: the one used longest ago
     goes, and a batch shape that comes back is captured again with the same tokens."""
